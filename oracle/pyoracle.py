@@ -18,6 +18,8 @@ REPO = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "liboracle.so")
 # the reference source tree the oracle builds compile; DISCO_REF overrides it
 REF_SRC = os.environ.get("DISCO_REF", "/root/reference")
+if not os.path.exists(os.path.join(REF_SRC, "paul.h")):
+    REF_SRC = os.path.join(REF_SRC, "absent")      # a directory without the sources is no tree
 
 
 def build_oracle(force=False):
