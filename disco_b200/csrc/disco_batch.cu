@@ -478,6 +478,7 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
    for( int d=0 ; d<ndisk ; ++d ) if( params[d].visc_flag ) b->any_visc = 1;
    b->gr = gr ? 1 : 0;
    b->d_zg_pairs = NULL;
+   b->d_zg_chains = NULL;
    b->zg_smem = 0;
    b->nq = mods->analysis == DISCO_DIAG_DISK2D ? 5 : mods->analysis == DISCO_DIAG_EULER ? 8 :
            mods->analysis == DISCO_DIAG_MHDMRI ? 18 : 0;
@@ -635,35 +636,40 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
          return (unsigned char)(s | ((m == SIDE_ZG_DIODE || m == SIDE_ZG_DIODE_PHIWIN) ? 4 : 0) |
                                 (side_mirror(m) ? 8 : 0) | (m == SIDE_NOSLIP ? 16 : 0));
       };
-      int maxr = 0, maxz = 0;
+      /* a chain: the ghost layers of one side of one column, from the real
+       * cells outwards */
+      auto pair_of = [&](int ghost, int src, unsigned char fl){
+         b->zg_pairs.push_back(make_int2(ghost, src)); b->zg_side.push_back(fl);
+      };
+      auto close = [&](size_t first){
+         if( b->zg_pairs.size() > first )
+            b->zg_chains.push_back(make_int2((int)first, (int)(b->zg_pairs.size() - first)));
+      };
+      b->zg_off.push_back(0);
       for( int d=0 ; d<ndisk ; ++d ){
          const DiskParams &D = b->dparams[d];
-         maxr = std::max(maxr, std::max(D.NgRa, D.NgRb));
-         if( D.Nz > 1 && !params[d].Z_Periodic ) maxz = std::max(maxz, std::max(D.NgZa, D.NgZb));
-      }
-      for( int l=0 ; l<maxr ; ++l ){
-         b->zg_off.push_back((int)b->zg_pairs.size());
-         for( int d=0 ; d<ndisk ; ++d ){
-            const DiskParams &D = b->dparams[d];
-            for( int k=0 ; k<D.Nz ; ++k ){
-               int base = D.ann0 + D.Nr*k;
-               /* a z ghost layer of a fixed z side ends fixed (the z pass runs
-                * after the r copies), so its r ghosts need no copy */
-               if( (k < D.NgZa && smode[2] == SIDE_FIXED) || (k >= D.Nz - D.NgZb && smode[3] == SIDE_FIXED) )
-                  continue;
-               if( l < D.NgRa && side_copies(smode[0]) ){
-                  int j = D.NgRa-1-l, j1 = side_mirror(smode[0]) ? 2*D.NgRa-j-1 : j+1;
-                  b->zg_pairs.push_back(make_int2(base+j, base+j1)); b->zg_side.push_back(flags(0));
-               }
-               if( l < D.NgRb && side_copies(smode[1]) ){
-                  int j = D.Nr-D.NgRb+l, j1 = side_mirror(smode[1]) ? 2*(D.Nr-D.NgRb)-j-1 : j-1;
-                  b->zg_pairs.push_back(make_int2(base+j, base+j1)); b->zg_side.push_back(flags(1));
-               }
+         for( int k=0 ; k<D.Nz ; ++k ){
+            int base = D.ann0 + D.Nr*k;
+            /* a z ghost layer of a fixed z side ends fixed (the z pass runs
+             * after the r copies), so its r ghosts need no copy */
+            if( (k < D.NgZa && smode[2] == SIDE_FIXED) || (k >= D.Nz - D.NgZb && smode[3] == SIDE_FIXED) )
+               continue;
+            size_t first = b->zg_pairs.size();
+            if( side_copies(smode[0]) ) for( int l=0 ; l<D.NgRa ; ++l ){
+               int j = D.NgRa-1-l, j1 = side_mirror(smode[0]) ? 2*D.NgRa-j-1 : j+1;
+               pair_of(base+j, base+j1, flags(0));
             }
+            close(first);
+            first = b->zg_pairs.size();
+            if( side_copies(smode[1]) ) for( int l=0 ; l<D.NgRb ; ++l ){
+               int j = D.Nr-D.NgRb+l, j1 = side_mirror(smode[1]) ? 2*(D.Nr-D.NgRb)-j-1 : j-1;
+               pair_of(base+j, base+j1, flags(1));
+            }
+            close(first);
          }
       }
       if( smode[1] == SIDE_ZG_DIODE_PHIWIN ){
-         b->zg_off.push_back((int)b->zg_pairs.size());
+         b->zg_off.push_back((int)b->zg_chains.size());
          for( int d=0 ; d<ndisk ; ++d ){
             const DiskParams &D = b->dparams[d];
             for( int k=0 ; k<D.Nz ; ++k ){
@@ -671,31 +677,33 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
                   continue;
                for( int j=D.Nr-D.NgRb ; j<D.Nr ; ++j ){
                   int A = D.ann0 + j + D.Nr*k;
-                  b->zg_pairs.push_back(make_int2(A, A)); b->zg_side.push_back((unsigned char)(1 | 32));
+                  size_t first = b->zg_pairs.size();
+                  pair_of(A, A, (unsigned char)(1 | 32));
+                  close(first);
                }
             }
          }
       }
-      for( int l=0 ; l<maxz ; ++l ){
-         b->zg_off.push_back((int)b->zg_pairs.size());
-         for( int d=0 ; d<ndisk ; ++d ){
-            const DiskParams &D = b->dparams[d];
-            if( D.Nz < 2 || params[d].Z_Periodic ) continue;
-            for( int j=0 ; j<D.Nr ; ++j ){
-               if( l < D.NgZa && side_copies(smode[2]) ){
-                  int k = D.NgZa-1-l, k1 = side_mirror(smode[2]) ? 2*D.NgZa-k-1 : k+1;
-                  b->zg_pairs.push_back(make_int2(D.ann0 + j + D.Nr*k, D.ann0 + j + D.Nr*k1));
-                  b->zg_side.push_back(flags(2));
-               }
-               if( l < D.NgZb && side_copies(smode[3]) ){
-                  int k = D.Nz-D.NgZb+l, k1 = side_mirror(smode[3]) ? 2*(D.Nz-D.NgZb)-k-1 : k-1;
-                  b->zg_pairs.push_back(make_int2(D.ann0 + j + D.Nr*k, D.ann0 + j + D.Nr*k1));
-                  b->zg_side.push_back(flags(3));
-               }
+      b->zg_off.push_back((int)b->zg_chains.size());
+      for( int d=0 ; d<ndisk ; ++d ){
+         const DiskParams &D = b->dparams[d];
+         if( D.Nz < 2 || params[d].Z_Periodic ) continue;
+         for( int j=0 ; j<D.Nr ; ++j ){
+            size_t first = b->zg_pairs.size();
+            if( side_copies(smode[2]) ) for( int l=0 ; l<D.NgZa ; ++l ){
+               int k = D.NgZa-1-l, k1 = side_mirror(smode[2]) ? 2*D.NgZa-k-1 : k+1;
+               pair_of(D.ann0 + j + D.Nr*k, D.ann0 + j + D.Nr*k1, flags(2));
             }
+            close(first);
+            first = b->zg_pairs.size();
+            if( side_copies(smode[3]) ) for( int l=0 ; l<D.NgZb ; ++l ){
+               int k = D.Nz-D.NgZb+l, k1 = side_mirror(smode[3]) ? 2*(D.Nz-D.NgZb)-k-1 : k-1;
+               pair_of(D.ann0 + j + D.Nr*k, D.ann0 + j + D.Nr*k1, flags(3));
+            }
+            close(first);
          }
       }
-      b->zg_off.push_back((int)b->zg_pairs.size());
+      b->zg_off.push_back((int)b->zg_chains.size());
       size_t sm = 0;
       for( const int2 &pr : b->zg_pairs ){
          size_t n0 = b->ann_np[pr.x], n1 = b->ann_np[pr.y];
@@ -800,6 +808,7 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
    }
    if( b->bc_zerograd && !b->zg_pairs.empty() ){
       b->d_zg_pairs = dupload(b, b->zg_pairs);
+      b->d_zg_chains = dupload(b, b->zg_chains);
       b->d_zg_side = dupload(b, b->zg_side);
    }
    make_float_view(b);

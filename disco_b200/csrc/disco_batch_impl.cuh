@@ -24,14 +24,15 @@ struct disco_batch {
    int any_mm3;
    int any_3d;               /* some disk has Nz > 1: z faces, gradz, z fluxes */
    int bc_zerograd;          /* Boundary/zerograd.c */
-   std::vector<int2> zg_pairs;          /* (ghost annulus, source annulus), by layer */
+   std::vector<int2> zg_pairs;          /* (ghost annulus, source annulus), chain by chain */
+   std::vector<int2> zg_chains;         /* (first pair, pairs): a side's layers, in order */
    std::vector<unsigned char> zg_side;  /* per pair: 0 inner r, 1 outer r, 2 lower z, 3 upper z */
    unsigned char *d_zg_side;
    int zg_diode, zg_omk;                /* outflow diode; Omega from initial() in r ghosts */
    int any_visc;                        /* some disk has Use_Viscosity (Euler) */
    int gr;                              /* HYDRO = grmhd2 (FP64, no constrained transport) */
-   std::vector<int> zg_off;             /* layer groups: r layers, a window layer, then z layers */
-   int2 *d_zg_pairs;
+   std::vector<int> zg_off;             /* chain groups: r layers, window entries, then z layers */
+   int2 *d_zg_pairs, *d_zg_chains;
    size_t zg_smem;                      /* dynamic shared memory of k_zerograd */
    std::vector<int2> zpole;             /* 3D CT z-pole annuli (annulus, 0 bottom / 1 top) */
    int2 *d_zpole;
@@ -100,16 +101,17 @@ static inline void mark(disco_batch *b, const char *name){
    b->tape_names->push_back(name);
 }
 
-/* boundary_trans of Boundary/zerograd.c (r layers, then z layers, each
- * layer from the real cells outwards), onestep.c:196-222 and main.c:53-62 */
+/* boundary_trans of Boundary/zerograd.c (the r layers, then the z layers, one
+ * launch each: a side's layers are one block's chain, from the real cells
+ * outwards), onestep.c:196-222 and main.c:53-62 */
 template<int Q, class R>
 static void launch_zerograd(disco_batch *b, const ViewT<R> &v){
    if( !b->bc_zerograd ) return;
    for( size_t g=0 ; g+1<b->zg_off.size() ; ++g ){
       int n = b->zg_off[g+1] - b->zg_off[g];
-      if( n > 0 ) k_zerograd<Q,R><<<n, 128, b->zg_smem, b->stream>>>(v, b->d_zg_pairs + b->zg_off[g],
-                                                                     b->d_zg_side + b->zg_off[g],
-                                                                     b->zg_diode, b->zg_omk);
+      if( n > 0 ) k_zerograd<Q,R><<<n, ZG_T, b->zg_smem, b->stream>>>(v, b->d_zg_chains + b->zg_off[g],
+                                                                      b->d_zg_pairs, b->d_zg_side,
+                                                                      b->zg_diode, b->zg_omk);
    }
    mark(b, "k_zerograd");
 }

@@ -1728,12 +1728,16 @@ __device__ __forceinline__ int zg_walk(const double *sp, const double *sd, const
 /* ------------------------------------------------------------------ zerograd
  * boundary_zerograd_{rinn,rout,zbot,ztop} (boundary_functions.c:269-440):
  * a ghost annulus takes the phi-overlap-weighted average of the adjacent
- * annulus (set_cells_copy_distant, :90-158).  One block per (ghost, source)
- * annulus pair of one layer: thread 0 replays the reference's traversal on
- * the two annuli's edges in shared memory and records, per ghost cell, the
- * source cell it starts from and how many it visits; then every thread sums
- * its ghost cell's overlaps in that order and divides by its dphi.  Loops
- * are capped; a cap hit raises ERRF_WRAP.  sides[] names each pair's
+ * annulus (set_cells_copy_distant, :90-158).  One block per chain of
+ * (ghost, source) annulus pairs, the ghost layers of one side of one r or z
+ * column in order from the real cells outwards (a layer's source is the
+ * layer before it, so the block's own barrier orders them and the layers
+ * need no launch each).  Per pair the reference's traversal of the two
+ * annuli's edges is replayed in shared memory, every thread walking its own
+ * ghost cells (below), which records per ghost cell the source cell it
+ * starts from and how many it visits; then every thread sums its ghost
+ * cells' overlaps in that order and divides by their dphi.  Loops are
+ * capped; a cap hit raises ERRF_WRAP.  sides[] names each pair's
  * boundary (0 inner r, 1 outer r, 2 lower z, 3 upper z); with `diode` the
  * copied normal velocity may only point out of the domain (the diode
  * argument of the same functions, used by outflow3d, zerograd_omk and
@@ -1741,18 +1745,24 @@ __device__ __forceinline__ int zg_walk(const double *sp, const double *sd, const
  * module (boundary_fixed_q_rinn / _rout with q = UPP, :662-718,
  * set_cell_init_q :33-47; zerograd_omk).  Higher bits of sides[]: 4 the
  * diode on this side only, 8 a mirror copy (boundary_reflect_*), 16 no-slip
- * (boundary_noslip_*, :914-1100), 32 a window-only entry with no copy. */
+ * (boundary_noslip_*, :914-1100), 32 a window-only entry with no copy.
+ *
+ * The kernel is a chain of shared-memory latencies, not of bytes: the walk
+ * is sequential in the reference, each ghost cell starting where the one
+ * before it stopped.  Walked by 32 lanes in runs, with a launch per layer, it
+ * took 120 of the 428 us of a 41 x 25-annulus MHD step; so split, the step
+ * takes 375 us (64 x 64 annuli: 3.02 -> 2.95 ms). */
+#define ZG_T 256
+#define ZG_ERR 0x40000000      /* in cnt[]: the cell's walk hit its cap */
 template<int Q, class R>
-__global__ void k_zerograd(ViewT<R> v, const int2 *pairs, const unsigned char *sides, int diode,
-                           int omk){
-   extern __shared__ __align__(16) unsigned char zg_smem[];
-   int2 pr = pairs[blockIdx.x];
+__device__ __forceinline__ void zerograd_pair(const ViewT<R> &v, int2 pr, int sflags, int diode, int omk,
+                                              unsigned char *zg_smem){
    const int a = pr.x, a1 = pr.y;
    const int np = v.ann_np[a], np1 = v.ann_np[a1];
    const int c0 = v.ann_off[a], c10 = v.ann_off[a1];
    const DiskParams &P = v.dp[v.ann_disk[a]];
    const double Pmax = P.Pmax;
-   if( sides[blockIdx.x] & 32 ){
+   if( sflags & 32 ){
       /* boundary_fixed_phi_rout(0.3 pi, 1.7 pi) (boundary_functions.c:809-843)
        * on a ghost annulus whose copies are all done (flowthrough.c:10-12):
        * set_cell_init on the cells whose centre lies in the window, no copy */
@@ -1782,7 +1792,7 @@ __global__ void k_zerograd(ViewT<R> v, const int2 *pairs, const unsigned char *s
    double *sd1 = sp1 + np1;
    int *st = reinterpret_cast<int*>(sd1 + np1);              /* start, count */
    int *cnt = st + np;
-   __shared__ int s_first;
+   __shared__ int s_first, s_bad;
    for( int i=threadIdx.x ; i<np ; i+=blockDim.x ){ sp[i] = v.piph[c0+i]; sd[i] = v.dphi[c0+i]; }
    for( int i=threadIdx.x ; i<np1 ; i+=blockDim.x ){ sp1[i] = v.piph[c10+i]; sd1[i] = v.dphi[c10+i]; }
    __shared__ int s_rot;
@@ -1806,29 +1816,25 @@ __global__ void k_zerograd(ViewT<R> v, const int2 *pairs, const unsigned char *s
    }
    __syncthreads();
    /* The walk of set_cells_copy_distant: ghost cell i starts at source cell
-    * st[i] and visits cnt[i] cells; the next starts where it stopped.  Warp 0
-    * splits the ghost cells into 32 runs; lane l walks run l from a guess of
-    * its start (the source cell holding the upper edge of the cell before
-    * the run).  Then each guess is checked against the end of the previous
-    * run; from the first wrong guess on, lane 0 walks the rest again, so
-    * st/cnt are those of the sequential walk in every case. */
-   if( threadIdx.x < 32 ){
-      const int lane = threadIdx.x;
-      const int seg = (np + 31)/32;
-      const int lo = lane*seg, hi = lo + seg < np ? lo + seg : np;
-      __shared__ int s_guess[32], s_end[32], s_err[32];
-      int err = 0, werr = 0;
-      int start = -1;
-      if( lo < np ){
-         if( lane == 0 ){
+    * st[i] and visits cnt[i] cells; the next starts at the last of them.
+    * Every thread walks its cells from a guess of their start (the source
+    * cell holding the upper edge of the cell before); a guess that the cell
+    * before does not end at is walked again in order, so st / cnt are those
+    * of the sequential walk in every case.  (32 runs walked by one warp, as
+    * before, left a dependent chain of np/32 cells.) */
+   if( threadIdx.x == 0 ) s_bad = np;
+   {
+      const int rot = s_rot;
+      for( int i=threadIdx.x ; i<np ; i+=blockDim.x ){
+         int start;
+         if( i == 0 ){
             start = s_first < np1 ? s_first : 0;
          }else{
-            /* a guess only (checked below): the source cell whose edge is
-             * the first at or after the upper edge of the cell before the
-             * run, by binary search over the source edges unrolled from
-             * the smallest; past the largest it is the cell that wraps */
-            const double pt = sp[lo-1];
-            const int rot = s_rot;
+            /* the source cell whose edge is the first at or after the upper
+             * edge of the cell before, by binary search over the source
+             * edges unrolled from the smallest; past the largest it is the
+             * cell that wraps */
+            const double pt = sp[i-1];
             int l0 = 0, h0 = np1;
             while( l0 < h0 ){
                int mid = (l0 + h0) >> 1;
@@ -1838,31 +1844,39 @@ __global__ void k_zerograd(ViewT<R> v, const int2 *pairs, const unsigned char *s
             start = rot + (l0 < np1 ? l0 : 0);
             if( start >= np1 ) start -= np1;
          }
+         int werr = 0;
+         zg_walk(sp, sd, sp1, sd1, np1, Pmax, i, i+1, start, st, cnt, &werr);
+         if( werr ) cnt[i] |= ZG_ERR;    /* counts only if this start is confirmed */
       }
-      s_guess[lane] = start;
-      int endi = -1;
-      if( lo < np && start >= 0 ) endi = zg_walk(sp, sd, sp1, sd1, np1, Pmax, lo, hi, start, st, cnt, &werr);
-      s_end[lane] = endi;
-      s_err[lane] = werr;           /* counts only if this run's start is confirmed */
-      __syncwarp();
-      if( lane == 0 ){
-         int bad = 32;
-         for( int l=1 ; l<32 && l*seg < np ; ++l )
-            if( s_guess[l] < 0 || s_guess[l] != s_end[l-1] ){ bad = l; break; }
-         for( int l=0 ; l<bad ; ++l ) err |= s_err[l];
-         if( bad < 32 ) zg_walk(sp, sd, sp1, sd1, np1, Pmax, bad*seg, np, s_end[bad-1], st, cnt, &err);
-      }
-      raise_err(v, err);
    }
    __syncthreads();
+   /* the cell a walk of n cells from s ends at */
+   auto end_of = [&](int s, int n){ return (s + (n & ~ZG_ERR) - 1) % np1; };
+   for( int i=threadIdx.x+1 ; i<np ; i+=blockDim.x )
+      if( st[i] != end_of(st[i-1], cnt[i-1]) ){ atomicMin(&s_bad, i); break; }
+   __syncthreads();
+   if( s_bad < np ){
+      if( threadIdx.x == 0 ){
+         for( int i=s_bad, e=end_of(st[i-1], cnt[i-1]) ; i<np ; ++i ){
+            if( st[i] != e ){
+               int werr = 0;
+               zg_walk(sp, sd, sp1, sd1, np1, Pmax, i, i+1, e, st, cnt, &werr);
+               if( werr ) cnt[i] |= ZG_ERR;
+            }
+            e = end_of(st[i], cnt[i]);
+         }
+      }
+      __syncthreads();
+   }
    const int N = v.Ncell;
    for( int i=threadIdx.x ; i<np ; i+=blockDim.x ){
       double phip = sp[i], phim = sp[i] - sd[i];
       double acc[Q];
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ) acc[q] = 0.0;
-      int i1 = st[i];
-      for( int n=0 ; n<cnt[i] ; ++n ){
+      int i1 = st[i], visits = cnt[i];
+      if( visits & ZG_ERR ){ raise_err(v, ERRF_WRAP); visits &= ~ZG_ERR; }
+      for( int n=0 ; n<visits ; ++n ){
          double phip1 = sp1[i1], phim1 = sp1[i1] - sd1[i1];
          int w = 0;
          while( phip1 < phim && w <= WRAP_CAP ){ phip1 += Pmax; phim1 += Pmax; ++w; }
@@ -1876,7 +1890,6 @@ __global__ void k_zerograd(ViewT<R> v, const int2 *pairs, const unsigned char *s
       }
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ) acc[q] = acc[q]/sd[i];
-      const int sflags = sides[blockIdx.x];
       const int side = sflags & 3;
       R out[Q];
 #pragma unroll
@@ -1905,6 +1918,16 @@ __global__ void k_zerograd(ViewT<R> v, const int2 *pairs, const unsigned char *s
       }
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ) v.prim[q*N + c0 + i] = out[q];
+   }
+}
+template<int Q, class R>
+__global__ void __launch_bounds__(ZG_T) k_zerograd(ViewT<R> v, const int2 *chains, const int2 *pairs,
+                                                   const unsigned char *sides, int diode, int omk){
+   extern __shared__ __align__(16) unsigned char zg_smem[];
+   const int2 ch = chains[blockIdx.x];
+   for( int p=ch.x ; p<ch.x+ch.y ; ++p ){
+      zerograd_pair<Q,R>(v, pairs[p], sides[p], diode, omk, zg_smem);
+      __syncthreads();        /* the next layer reads this one's prims */
    }
 }
 
