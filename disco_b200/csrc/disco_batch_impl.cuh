@@ -195,7 +195,7 @@ static void launch_flux_t(disco_batch *b, const ViewT<R> &v0){
 
 /* One substep of onestep() (onestep.c:84-229); GR: the grmhd2 module. */
 template<int Q, int NC, class R, bool GR = false>
-static void launch_substep(disco_batch *b, ViewT<R> v, double RK, int first, int last, double dtfac){
+static void launch_substep(disco_batch *b, ViewT<R> v, int first, int last, double dtfac){
    v.dtfac = dtfac;
    /* RK2: the first substep keeps the faces the previous step's second
     * substep built from the same piph; that substep marks them valid */
@@ -204,7 +204,7 @@ static void launch_substep(disco_batch *b, ViewT<R> v, double RK, int first, int
    v.move_c2p = first && !b->ct;
    cudaStream_t s = b->stream;
    unsigned ncb = (unsigned)b->cblk.size(), nfb = (unsigned)b->fblk.size();
-   k_begin<Q,NC,R,GR><<<ncb, CB, 0, s>>>(v, RK, first);               mark(b, "k_begin");
+   k_begin<Q,NC,R,GR><<<ncb, CB, 0, s>>>(v, first);                   mark(b, "k_begin");
    if( first && b->any_mm3 ){ k_wmean<R><<<nblk(v.Nann, WM_WARPS), 32*WM_WARPS, 0, s>>>(v, 1); mark(b, "k_wmean"); }
    k_I0<R><<<nblk((size_t)v.Nann*32, 128), 128, 0, s>>>(v);           mark(b, "k_I0");
    {  /* the same blocks in the order that keeps an annulus's three tracks together */
@@ -303,12 +303,12 @@ static void launch_step_qt(disco_batch *b, const ViewT<R> &v, int use_next){
    unsigned nd = nblk(b->ndisk, 64);
    k_disk_begin<R><<<nd, 64, 0, s>>>(v, b->ndisk, use_next);          mark(b, "k_disk_begin");
    if( b->timestep_mode == 1 ){
-      launch_substep<Q,NC,R,GR>(b, v, 0.0, 1, 1, 1.0);
+      launch_substep<Q,NC,R,GR>(b, v, 1, 1, 1.0);
       k_disk_mid<R><<<nd, 64, 0, s>>>(v, b->ndisk, 0.0, 1, 1);       mark(b, "k_disk_mid");
    }else{
-      launch_substep<Q,NC,R,GR>(b, v, 0.0, 1, 0, 1.0);
+      launch_substep<Q,NC,R,GR>(b, v, 1, 0, 1.0);
       k_disk_mid<R><<<nd, 64, 0, s>>>(v, b->ndisk, 0.0, 1, 1);       mark(b, "k_disk_mid");
-      launch_substep<Q,NC,R,GR>(b, v, 0.5, 0, 1, 0.5);
+      launch_substep<Q,NC,R,GR>(b, v, 0, 1, 0.5);
       k_disk_mid<R><<<nd, 64, 0, s>>>(v, b->ndisk, 0.5, 0, 0);       mark(b, "k_disk_mid");
    }
    if( b->nq ){

@@ -214,12 +214,14 @@ __device__ __forceinline__ void acc(double &s, double &cc, double x){
 }
 
 /* ------------------------------------------------------------------ k_begin
- * First substep: RK snapshot (timestep.c:18-24), set_wcell (misc.c:101-168,
- * modes 0/1/2/4; mode 3's mean is k_wmean), the moved-and-wrapped piph of
- * move_cells + clean_pi (misc.c:256-268, 8-26) into piph_new.
- * Every substep: adjust_RK_cons (misc.c:226-244) and plm_phi (plm.c:15-51). */
+ * First substep: set_wcell (misc.c:101-168, modes 0/1/2/4; mode 3's mean is
+ * k_wmean), the moved-and-wrapped piph of move_cells + clean_pi (misc.c:
+ * 256-268, 8-26) into piph_new.  Every substep: plm_phi (plm.c:15-51).
+ * The RK snapshot and average (timestep.c:18-24, adjust_RK_cons misc.c:
+ * 226-244) are taken where cons and Phi are read next, in k_update and
+ * k_ct_update: nothing in between reads them. */
 template<int Q, int NC, class R, bool GR = false>
-__device__ __forceinline__ void begin_body(const ViewT<R> &v, double RK, int first, int bid){
+__device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid){
    /* the chunk's prims and dphi staged once, with one neighbour cell on each
     * side (slot t+1 = cell i0+t) */
    __shared__ R sp[Q][CB+2];
@@ -281,33 +283,6 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, double RK, int fir
          raise_err(v, err);
       }
    }
-#pragma unroll
-   for( int q=0 ; q<Q ; ++q ){
-      double cq = v.cons[q*N + c];
-      double rk;
-      if( first ){ rk = cq; v.RKcons[q*N + c] = cq; }
-      else rk = v.RKcons[q*N + c];
-      /* with RK = 0 (the first substep) the average returns a finite cq
-       * bit for bit, so the store is skipped */
-      if( !(RK == 0.0 && isfinite(cq)) ) v.cons[q*N + c] = (1.-RK)*cq + RK*rk;
-      if constexpr ( sizeof(R) != sizeof(double) ){
-         /* the carry belongs to cons; averaged with it (RKcons keeps none) */
-         if( !first ) v.ccarry[q*N + c] = (float)((1.-RK)*(double)v.ccarry[q*N + c]);
-      }
-   }
-   if constexpr ( NC == 8 ){
-      if( v.ct ){                   /* timestep.c:22 and adjust_RK_cons, misc.c:239-241 */
-#pragma unroll
-         for( int s=0 ; s<5 ; ++s ){
-            if( s >= v.nfs ) break;
-            double ph = v.Phi[s*N + c];
-            double rk;
-            if( first ){ rk = ph; v.RKPhi[s*N + c] = ph; }
-            else rk = v.RKPhi[s*N + c];
-            if( !(RK == 0.0 && isfinite(ph)) ) v.Phi[s*N + c] = (1.-RK)*ph + RK*rk;
-         }
-      }
-   }
    const R dpL = (R)sd[t], dpC = (R)sd[t+1], dpR = (R)sd[t+2];
    const R PLM = (R)P.PLM;
 #pragma unroll
@@ -325,8 +300,8 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, double RK, int fir
    }
 }
 template<int Q, int NC, class R, bool GR = false>
-__global__ void __launch_bounds__(CB, GR ? MB_GR_LIGHT : (Q > 6 ? MB_MHD_BEGIN : MB_BEGIN)) k_begin(ViewT<R> v, double RK, int first){
-   begin_body<Q,NC,R,GR>(v, RK, first, blockIdx.x);
+__global__ void __launch_bounds__(CB, GR ? MB_GR_LIGHT : (Q > 6 ? MB_MHD_BEGIN : MB_BEGIN)) k_begin(ViewT<R> v, int first){
+   begin_body<Q,NC,R,GR>(v, first, blockIdx.x);
 }
 
 /* Energy-frame Omega at the radii the step evaluates it (omega.c:62-110):
@@ -980,8 +955,24 @@ __device__ __forceinline__ QVec<Q,R> phi_face_flux_visc(const ViewT<R> &v, const
    return G;
 }
 
+/* The RK snapshot of the first substep (timestep.c:18-24: RK_x = x) or the
+ * average of the second (adjust_RK_cons, misc.c:226-244, RK = 1/2), element
+ * o of x; returns the value the substep's update starts from.  In the first
+ * (RK = 0) that is x itself, bit for bit, unless x is not finite. */
+__device__ __forceinline__ double rk_start(const double *x, double *RKx, size_t o, int first){
+   const double xo = x[o];
+   if( first ){
+      RKx[o] = xo;
+      return isfinite(xo) ? xo : xo + 0.0*xo;
+   }
+   return (1.-.5)*xo + .5*RKx[o];
+}
+
 /* ------------------------------------------------------------------ k_update
  * The flux gather and sources, per cell, in the reference's order:
+ *   RK snapshot / average  of cons (rk_start), as its one read of cons
+ *                (a pass of its own over cons in k_begin, it cost the ragged64
+ *                step 0.11 ms of 5.4, download included)
  *   flux gather  riemann.c:312-315 applied as phi_flux then trans_flux do
  *   add_source   misc.c:538-580 (euler source + planet_src), pre-move cell,
  *                FP64 in both forms (the disk's force balance)
@@ -1103,9 +1094,12 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       double cons[Q], cc[Q];
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ){
-         cons[q] = v.cons[q*N + c];
-         if constexpr ( sizeof(R) != sizeof(double) ) cc[q] = (double)v.ccarry[q*N + c];
-         else cc[q] = 0.0;
+         cons[q] = rk_start(v.cons, v.RKcons, (size_t)q*N + c, first);
+         if constexpr ( sizeof(R) != sizeof(double) ){
+            /* the carry belongs to cons; averaged with it (RKcons keeps none) */
+            cc[q] = (double)v.ccarry[q*N + c];
+            if( !first ) cc[q] = (double)(float)(.5*cc[q]);
+         }else cc[q] = 0.0;
       }
       /* The face fluxes: in the FP64 path added to cons one by one in the
        * reference's order; in the mixed form (FP32 fluxes) summed in a plain
@@ -1236,7 +1230,11 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
          if constexpr ( sizeof(R) != sizeof(double) ) v.ccarry[q*N + c] = (float)cc[q];
       }
    }
-   (void)first;                     /* the move follows in k_c2p (or k_ct_update) */
+   else if( first ){                /* a ghost's cons is not evolved: its snapshot alone */
+#pragma unroll
+      for( int q=0 ; q<Q ; ++q ) v.RKcons[q*N + c] = v.cons[q*N + c];
+   }
+   /* the move follows in k_c2p (or k_ct_update) */
    raise_err(v, err);
 }
 template<int Q, int NC, class R, bool VISC = false, bool GR = false>

@@ -224,7 +224,7 @@ __device__ __forceinline__ void persist_run(const ViewT<R> &v, const PersistArgs
    const double dtfac = sub ? 0.5 : 1.0;
    switch( stage ){
    case PS_DBEGIN:  if( tid == 0 ) disk_begin_body<R>(v, x, pa.use_next); break;
-   case PS_BEGIN:   begin_body<Q,NC,R>(v, sub ? 0.5 : 0.0, !sub, x); break;
+   case PS_BEGIN:   begin_body<Q,NC,R>(v, !sub, x); break;
    case PS_I0:      if( (tid >> 5) < n ) I0_body<R>(v, !sub, x + (tid >> 5), tid & 31); break;
    case PS_FACES:   faces_body<Q,R>(v, 1, !sub, x); break;
    case PS_GRAD:    grad_body<Q,1,R>(v, x); break;
