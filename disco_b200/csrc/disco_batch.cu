@@ -487,6 +487,8 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
    b->any_3d = 0;
    b->graph = NULL;
    b->have_cells = 0;
+   b->topo_known = 0;
+   b->own_capture = 0; b->general = 0;
    b->stream = NULL;
    b->own_stream = NULL;
    b->tape = NULL; b->tape_names = NULL;
@@ -617,8 +619,11 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
       }
    }
    if( b->fblk_rz.size() != b->fblk.size() ){ delete b; return DISCO_ERR_INTERNAL; }
-   for( const int2 &fb : b->fblk )
-      if( b->tr_flux[fb.x] ) b->fblk_fl[b->tr_dim[fb.x] - 1].push_back(fb);
+   for( int dim=1 ; dim<=2 ; ++dim ){
+      for( const int2 &fb : b->fblk )
+         if( b->tr_flux[fb.x] && b->tr_dim[fb.x] == dim ) b->fblk_fl.push_back(fb);
+      if( dim == 1 ) b->nfl_r = (int)b->fblk_fl.size();
+   }
 
    /* zerograd layers (boundary_functions.c:269-440): r ghosts from the real
     * cells outwards, then z ghosts (all j, ghosts included); sides[] of each
@@ -734,7 +739,7 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
    v.ann_rc = dupload(b, b->ann_rc);
    v.cblk = dupload(b, b->cblk); v.fblk = dupload(b, b->fblk); v.ublk = dupload(b, b->ublk);
    b->d_fblk_rz = dupload(b, b->fblk_rz);
-   b->d_fblk_fl[0] = dupload(b, b->fblk_fl[0]); b->d_fblk_fl[1] = dupload(b, b->fblk_fl[1]);
+   b->d_fblk_fl = dupload(b, b->fblk_fl);
    v.rj = dupload(b, b->rj); v.zk = dupload(b, b->zk);
    v.dp = dupload(b, b->dparams);
    v.ds = dupload(b, dstate);
@@ -982,6 +987,7 @@ extern "C" int disco_batch_set_cells(disco_batch *b, const double *prim, const d
    CK(xfer(b, b->vd.dphi, dphi, N*sizeof(double), cudaMemcpyHostToDevice));
    if( wiph ) CK(xfer(b, b->vd.wiph, wiph, N*sizeof(double), cudaMemcpyHostToDevice));
    if( b->vd.ccarry ) CK(cudaMemsetAsync(b->vd.ccarry, 0, (size_t)b->Q*N*sizeof(float), b->stream));
+   b->topo_known = 0;
    CK(cudaMemsetAsync(b->vd.topo, 0, sizeof(int), b->stream));      /* new piph: faces stale */
    if( prim && !cons ){
       unsigned ncb = (unsigned)b->cblk.size();
@@ -1042,6 +1048,7 @@ extern "C" int disco_batch_setup_cells(disco_batch *b){
    if( b->mods.initial == DISCO_IC_HOST ) return DISCO_ERR_UNSUPPORTED;   /* set up on the host */
    if( noise_missing(b) ) return DISCO_ERR_STATE;
    CK(cudaSetDevice(b->device));
+   b->topo_known = 0;
    CK(cudaMemsetAsync(b->vd.topo, 0, sizeof(int), b->stream));
    if( b->prec == DISCO_PREC_MIXED ) mixed_launch_setup(b);
    else launch_setup_t(b, b->vd);
@@ -1105,10 +1112,19 @@ extern "C" int disco_batch_run(disco_batch *b, int nsteps){
    if( !b || nsteps < 0 ) return DISCO_ERR_ARG;
    if( !b->have_cells ) return DISCO_ERR_STATE;
    CK(cudaSetDevice(b->device));
-   if( !b->graph ){
+   /* the captured step takes the kept faces as given: the first step after an
+    * upload, which builds them, is launched as it is */
+   if( nsteps > 0 && b->sched == DISCO_SCHED_KERNELS && b->timestep_mode == 0 && !b->topo_known ){
+      launch_step(b, 1);
+      CK(cudaGetLastError());
+      nsteps--;
+   }
+   if( !b->graph && nsteps > 0 ){
       cudaGraph_t g;
       CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+      b->own_capture = 1;
       launch_step(b, 1);
+      b->own_capture = 0;
       CK(cudaStreamEndCapture(b->stream, &g));
       CK(cudaGraphInstantiate(&b->graph, g, 0));
       CK(cudaGraphDestroy(g));
@@ -1197,6 +1213,7 @@ extern "C" int disco_batch_restart_cells(disco_batch *b, const double *prim, con
       CK(xfer(b, b->vd.Phi, t.data(), t.size()*sizeof(double), cudaMemcpyHostToDevice));
    }
    CK(xfer(b, b->vd.piph, piph, N*sizeof(double), cudaMemcpyHostToDevice));
+   b->topo_known = 0;
    CK(cudaMemsetAsync(b->vd.topo, 0, sizeof(int), b->stream));
    /* diagnostics restart from zero (h5in.c:329-333), as does the step count
     * of a new process (domain.c:99) */

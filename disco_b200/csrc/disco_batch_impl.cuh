@@ -48,8 +48,9 @@ struct disco_batch {
    std::vector<int2> cblk, fblk;
    /* the same face blocks in k_faces' order (per layer, the r and z tracks of
     * each annulus together) and the blocks k_flux_t solves per direction */
-   std::vector<int2> fblk_rz, fblk_fl[2];
-   int2 *d_fblk_rz, *d_fblk_fl[2];
+   std::vector<int2> fblk_rz, fblk_fl;
+   int2 *d_fblk_rz, *d_fblk_fl;
+   int nfl_r;                           /* of fblk_fl: r-track blocks, before the z-track ones */
    std::vector<int2> ublk;              /* k_update's blocks: chunks of CB-1 cells */
    std::vector<int> ann_blk0, ann_nblk;
    std::vector<double> rj, zk;
@@ -72,6 +73,8 @@ struct disco_batch {
    std::vector<const char *> *tape_names;
    cudaGraphExec_t graph;
    int have_cells;
+   int topo_known;           /* the device's topo flag is set once the queued work has run */
+   int own_capture, general; /* disco_batch_run is capturing; the step in flight runs every pass */
    int ct;                   /* constrained transport: the CT_MODE (1, 2) or 0 (FP64 view only) */
    int nfs;                  /* face-flux slots per cell (NUM_FACES: 3 or 5) */
    std::vector<int> line_off;           /* edge lines of 3D CT, offsets into lineX */
@@ -181,12 +184,14 @@ static void launch_c2p(disco_batch *b, const ViewT<R> &v, int last, int diag){
    if( b->nq == 8 ) launch_c2p_nq<Q,NC,R,8,GR>(b, v, last, diag);
    else launch_c2p_nq<Q,NC,R,5,GR>(b, v, last, diag);
 }
+/* trans_flux of one direction, only the blocks of its tracks with fluxes
+ * (one launch for both compiled the two solves into one register budget:
+ * the GRMHD step slowed by 6%) */
 template<int Q, int NC, int DIM, class R, bool GR = false>
 static void launch_flux_t(disco_batch *b, const ViewT<R> &v0){
-   /* only the blocks of this direction's tracks with trans_flux faces */
-   unsigned nfb = (unsigned)b->fblk_fl[DIM-1].size();
+   const unsigned nfb = DIM == 1 ? (unsigned)b->nfl_r : (unsigned)b->fblk_fl.size() - b->nfl_r;
    if( nfb == 0 ) return;
-   ViewT<R> v = v0; v.fblk = b->d_fblk_fl[DIM-1];
+   ViewT<R> v = v0; v.fblk = b->d_fblk_fl + (DIM == 1 ? 0 : b->nfl_r);
    if constexpr ( NC == 5 ){
       if( b->any_visc ){ k_flux_t<Q,NC,DIM,R,true><<<nfb, FB, 0, b->stream>>>(v); return; }
    }
@@ -200,21 +205,26 @@ static void launch_substep(disco_batch *b, ViewT<R> v, int first, int last, doub
    /* RK2: the first substep keeps the faces the previous step's second
     * substep built from the same piph; that substep marks them valid */
    v.topo_reuse = first && b->timestep_mode == 0;
+   /* I0 is not launched where the host knows the faces to be kept (the
+    * instrumented step runs every pass) */
+   const bool build = !(v.topo_reuse && b->topo_known) || b->tape || b->general;
    v.topo_set = !first;
    v.move_c2p = first && !b->ct;
    cudaStream_t s = b->stream;
    unsigned ncb = (unsigned)b->cblk.size(), nfb = (unsigned)b->fblk.size();
-   k_begin<Q,NC,R,GR><<<ncb, CB, 0, s>>>(v, first);                   mark(b, "k_begin");
-   if( first && b->any_mm3 ){ k_wmean<R><<<nblk(v.Nann, WM_WARPS), 32*WM_WARPS, 0, s>>>(v, 1); mark(b, "k_wmean"); }
-   k_I0<R><<<nblk((size_t)v.Nann*32, 128), 128, 0, s>>>(v);           mark(b, "k_I0");
+   const unsigned nI0 = build ? nblk((size_t)v.Nann, CB/32) : 0;
+   mark(b, "k_I0");                                    /* part of the next launch */
+   k_begin<Q,NC,R,GR><<<nI0 + nblk(b->ndisk, CB) + ncb, CB, 0, s>>>(v, first, (int)nI0, b->ndisk);
+   mark(b, "k_begin");
    {  /* the same blocks in the order that keeps an annulus's three tracks together */
       ViewT<R> vf = v; vf.fblk = b->d_fblk_rz;
       k_faces<Q,R><<<nfb, FB, 0, s>>>(vf, 1);                          mark(b, "k_faces");
    }
-   if( b->any_3d ){ k_grad_rz<Q,R><<<ncb, CB, 0, s>>>(v);             mark(b, "k_grad"); }
-   else{ k_grad<Q,1,R><<<ncb, CB, 0, s>>>(v);                         mark(b, "k_gradr"); }
-   launch_flux_t<Q,NC,1,R,GR>(b, v);                                  mark(b, "k_flux_r");
-   if( b->any_3d ){ launch_flux_t<Q,NC,2,R,GR>(b, v);                 mark(b, "k_flux_z"); }
+   const unsigned nwm = first && b->any_mm3 ? nblk(v.Nann, WM_WARPS) : 0;
+   if( b->any_3d ){ k_grad<Q,true,R><<<nwm + ncb, CB, 0, s>>>(v, (int)nwm);  mark(b, "k_grad"); }
+   else{            k_grad<Q,false,R><<<nwm + ncb, CB, 0, s>>>(v, (int)nwm); mark(b, "k_gradr"); }
+   launch_flux_t<Q,NC,1,R,GR>(b, v);                   mark(b, "k_flux_r");
+   if( b->any_3d ){ launch_flux_t<Q,NC,2,R,GR>(b, v);  mark(b, "k_flux_z"); }
    bool upd_visc = false;
    if constexpr ( NC == 5 ) upd_visc = b->any_visc;
    if( upd_visc ){
@@ -298,24 +308,27 @@ static int persist_blocks_per_sm_t(const disco_batch *b){
 /* timestep() (timestep.c:7-45). */
 template<int Q, int NC, class R, bool GR = false>
 static void launch_step_qt(disco_batch *b, const ViewT<R> &v, int use_next){
-   if( b->sched == DISCO_SCHED_PERSISTENT ){ launch_persist<Q,NC,R>(b, v, use_next); return; }
-   cudaStream_t s = b->stream;
-   unsigned nd = nblk(b->ndisk, 64);
-   k_disk_begin<R><<<nd, 64, 0, s>>>(v, b->ndisk, use_next);          mark(b, "k_disk_begin");
-   if( b->timestep_mode == 1 ){
-      launch_substep<Q,NC,R,GR>(b, v, 1, 1, 1.0);
-      k_disk_mid<R><<<nd, 64, 0, s>>>(v, b->ndisk, 0.0, 1, 1);       mark(b, "k_disk_mid");
-   }else{
+   if( b->sched == DISCO_SCHED_PERSISTENT ){
+      b->topo_known = 0;            /* a launch that timed out leaves no list */
+      launch_persist<Q,NC,R>(b, v, use_next);
+      return;
+   }
+   const bool fe = b->timestep_mode == 1;
+   /* a step that a caller captures may be replayed after an upload, and has
+    * not run when it is captured: every pass, and nothing learnt from it */
+   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+   cudaStreamIsCapturing(b->stream, &cap);
+   b->general = cap != cudaStreamCaptureStatusNone && !b->own_capture;
+   if( fe ) launch_substep<Q,NC,R,GR>(b, v, 1, 1, 1.0);
+   else{
       launch_substep<Q,NC,R,GR>(b, v, 1, 0, 1.0);
-      k_disk_mid<R><<<nd, 64, 0, s>>>(v, b->ndisk, 0.0, 1, 1);       mark(b, "k_disk_mid");
       launch_substep<Q,NC,R,GR>(b, v, 0, 1, 0.5);
-      k_disk_mid<R><<<nd, 64, 0, s>>>(v, b->ndisk, 0.5, 0, 0);       mark(b, "k_disk_mid");
+      if( !b->general ) b->topo_known = 1;
    }
-   if( b->nq ){
-      k_diag_finish<R><<<nblk(v.Nann, 128), 128, 0, s>>>(v, b->d_Qrz, b->d_ann_blk0, b->d_ann_nblk);
-      mark(b, "k_diag_finish");
-   }
-   k_disk_end<R><<<nd, 64, 0, s>>>(v, b->ndisk);                      mark(b, "k_disk_end");
+   const unsigned nx = (unsigned)(v.Nann > b->ndisk ? v.Nann : b->ndisk);
+   k_step_end<R><<<nblk(nx, 128), 128, 0, b->stream>>>(v, b->ndisk, fe ? 0.0 : 0.5, fe ? 1 : 0, fe ? 1 : 0,
+                                                       b->d_Qrz, b->d_ann_blk0, b->d_ann_nblk);
+   mark(b, "k_step_end");
 }
 
 /* Dispatch on the Hydro module: NUM_C 5 (euler) or 8 (mhd), NUM_N 1. */

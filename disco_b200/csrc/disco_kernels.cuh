@@ -275,7 +275,7 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid
       if( P.mesh_motion != 3 ){
          int err = 0;
          /* move_cells: never contracted to an FMA, so both forms move alike */
-         double phi = __dadd_rn(v.piph[c], __dmul_rn(w, v.ds[d].dt));
+         double phi = __dadd_rn(v.piph[c], __dmul_rn(w, v.ds[d].dt_next));   /* the step's dt */
          int n = 0;
          while( phi > P.Pmax ){ phi -= P.Pmax; if( ++n > WRAP_CAP ){ err |= ERRF_WRAP; break; } }
          while( phi < 0.0 ){ phi += P.Pmax; if( ++n > WRAP_CAP ){ err |= ERRF_WRAP; break; } }
@@ -299,11 +299,6 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid
       v.gradp[q*N + c] = m;
    }
 }
-template<int Q, int NC, class R, bool GR = false>
-__global__ void __launch_bounds__(CB, GR ? MB_GR_LIGHT : (Q > 6 ? MB_MHD_BEGIN : MB_BEGIN)) k_begin(ViewT<R> v, int first){
-   begin_body<Q,NC,R,GR>(v, first, blockIdx.x);
-}
-
 /* Energy-frame Omega at the radii the step evaluates it (omega.c:62-110):
  * annulus centroids (sources, phi faces, c2p) and r-faces (trans_flux). */
 template<class R>
@@ -350,30 +345,30 @@ __global__ void k_gr_tables(ViewT<R> v){
 }
 
 /* Mesh_Motion 3 (misc.c:138-152): annulus mean of w, summed in cell order
- * (one warp per annulus: lane 0 adds the values in cell order from shared
- * memory, the warp loads and writes), then the move of the first substep
- * (move != 0) or not (set-up). */
+ * (one warp per annulus: each lane loads a cell's value, and all lanes add
+ * the 32 values in cell order from the shuffles), then the move of the first
+ * substep (move != 0) or not (set-up). */
 #define WM_WARPS 4
-#define WM_CHUNK 256
 template<class R>
-__global__ void __launch_bounds__(32*WM_WARPS) k_wmean(ViewT<R> v, int move){
-   __shared__ double s_w[WM_WARPS][WM_CHUNK];
+__device__ __forceinline__ void wmean_body(const ViewT<R> &v, int move, int bid){
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int a = blockIdx.x*WM_WARPS + warp;
-   if( a >= v.Nann ) return;
+   const int a = bid*WM_WARPS + warp;
+   if( warp >= WM_WARPS || a >= v.Nann ) return;
    const int np = v.ann_np[a], c0 = v.ann_off[a];
    const int d = v.ann_disk[a];
    const DiskParams &P = v.dp[d];
    if( P.mesh_motion != 3 ) return;
    double w = 0.0;
-   for( int base=0 ; base<np ; base+=WM_CHUNK ){
-      const int n = np - base < WM_CHUNK ? np - base : WM_CHUNK;
-      for( int t=lane ; t<n ; t+=32 ) s_w[warp][t] = v.wiph[c0+base+t];
-      __syncwarp();
-      if( lane == 0 ) for( int t=0 ; t<n ; ++t ) w += s_w[warp][t];
-      __syncwarp();
+   double x = lane < np ? v.wiph[c0+lane] : 0.0;
+   for( int base=0 ; base<np ; base+=32 ){
+      const int n = np - base < 32 ? np - base : 32;
+      const double xn = base+32+lane < np ? v.wiph[c0+base+32+lane] : 0.0;
+      if( n == 32 ){
+#pragma unroll
+         for( int t=0 ; t<32 ; ++t ) w += __shfl_sync(0xffffffffu, x, t);
+      }else for( int t=0 ; t<n ; ++t ) w += __shfl_sync(0xffffffffu, x, t);
+      x = xn;
    }
-   w = __shfl_sync(0xffffffffu, w, 0);
    w /= (double)np;
    const double dt = v.ds[d].dt;
    int err = 0;
@@ -388,6 +383,11 @@ __global__ void __launch_bounds__(32*WM_WARPS) k_wmean(ViewT<R> v, int move){
       }
    }
    raise_err(v, err);
+}
+
+template<class R>
+__global__ void __launch_bounds__(32*WM_WARPS) k_wmean(ViewT<R> v, int move){
+   wmean_body<R>(v, move, blockIdx.x);
 }
 
 /* ------------------------------------------------------------------ k_I0
@@ -706,16 +706,16 @@ __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
    for( int q=0 ; q<Q ; ++q ) grad[q*N + c] = g[q];
    raise_err(v, err);
 }
-template<int Q, int DIM, class R>
-__global__ void __launch_bounds__(CB, Q > 6 ? MB_MHD_GRAD : MB_GRAD) k_grad(ViewT<R> v){
-   grad_body<Q,DIM,R>(v, blockIdx.x);
-}
-/* both directions of a 3D grid in one launch: the cell's annulus data are
- * read once and the two gathers' loads overlap */
-template<int Q, class R>
-__global__ void __launch_bounds__(CB, Q > 6 ? MB_MHD_GRAD : MB_GRAD) k_grad_rz(ViewT<R> v){
-   grad_body<Q,1,R>(v, blockIdx.x);
-   grad_body<Q,2,R>(v, blockIdx.x);
+/* The r direction, with D3 also the z direction of a 3D grid (the cell's
+ * annulus data are read once and the two gathers' loads overlap).  The first
+ * nwm blocks take the Mesh_Motion 3 mean of the first substep, which nothing
+ * reads before k_update. */
+template<int Q, bool D3, class R>
+__global__ void __launch_bounds__(CB, Q > 6 ? MB_MHD_GRAD : MB_GRAD) k_grad(ViewT<R> v, int nwm){
+   const int bid = (int)blockIdx.x - nwm;
+   if( bid < 0 ){ wmean_body<R>(v, 1, blockIdx.x); return; }
+   grad_body<Q,1,R>(v, bid);
+   if constexpr ( D3 ) grad_body<Q,2,R>(v, bid);
 }
 
 /* The viscous flux of a face, compiled only into the viscous instances of
@@ -1945,13 +1945,8 @@ __device__ __forceinline__ void disk_begin_body(const ViewT<R> &v, int d, int us
    if( dt0 <= 0.0 ) dt0 = 1.0e100;
    S.dtmin = dbits(dt0);
 }
-template<class R>
-__global__ void k_disk_begin(ViewT<R> v, int ndisk, int use_next){
-   int d = blockIdx.x*blockDim.x + threadIdx.x;
-   if( d < ndisk ) disk_begin_body<R>(v, d, use_next);
-}
-
-/* cos / sin of the planets' phi at set-up (later kept by k_disk_begin/mid) */
+/* cos / sin of the planets' phi at set-up (later kept by disk_begin_body /
+ * disk_mid_body) */
 template<class R>
 __global__ void k_planet_trig(ViewT<R> v, int ndisk){
    int d = blockIdx.x*blockDim.x + threadIdx.x;
@@ -1991,12 +1986,6 @@ __device__ __forceinline__ void disk_mid_body(const ViewT<R> &v, int d, double R
    }
    if( advance_t ) S.t += dt;
 }
-template<class R>
-__global__ void k_disk_mid(ViewT<R> v, int ndisk, double RK, int first, int advance_t){
-   int d = blockIdx.x*blockDim.x + threadIdx.x;
-   if( d < ndisk ) disk_mid_body<R>(v, d, RK, first, advance_t);
-}
-
 /* End of timestep(): dt of the next step, diagnostics time (analysis.c:105),
  * count_steps. */
 template<class R>
@@ -2010,12 +1999,6 @@ __device__ __forceinline__ void disk_end_body(const ViewT<R> &v, int d){
    if( !(S.dt_next > 0.0) || S.dt_next != S.dt_next || S.dt_next >= 1.0e99 )
       atomicOr(v.err, ERRF_NONFINITE);
 }
-template<class R>
-__global__ void k_disk_end(ViewT<R> v, int ndisk){
-   int d = blockIdx.x*blockDim.x + threadIdx.x;
-   if( d < ndisk ) disk_end_body<R>(v, d);
-}
-
 /* Per annulus: sum its blocks' diagnostic partials in block order. */
 template<class R>
 __device__ __forceinline__ void diag_finish_body(const ViewT<R> &v, double *Qrz, const int *ann_blk0,
@@ -2030,10 +2013,44 @@ __device__ __forceinline__ void diag_finish_body(const ViewT<R> &v, double *Qrz,
    }
    for( int m=0 ; m<nq ; ++m ) Qrz[(size_t)a*nq + m] += s[m]*dt / s[DIAG_VOL];
 }
+
+/* ------------------------------------------------------------------ k_begin
+ * A substep's first launch: the cells' begin_body, and beside it what needs
+ * no launch of its own -- the annuli's I0 (nI0 blocks; piph is not written
+ * here) and per disk the start of timestep() (first substep) or the planets'
+ * update after the first substep (second).  On a disk of a few blocks the
+ * step is a chain of launches of 3-5 us each, so each one folded away shows. */
+template<int Q, int NC, class R, bool GR = false>
+__global__ void __launch_bounds__(CB, GR ? MB_GR_LIGHT : (Q > 6 ? MB_MHD_BEGIN : MB_BEGIN))
+k_begin(ViewT<R> v, int first, int nI0, int ndisk){
+   const int nd = (ndisk + CB - 1)/CB;
+   const int bid = (int)blockIdx.x - nI0 - nd;
+   if( bid >= 0 ){
+      begin_body<Q,NC,R,GR>(v, first, bid);
+      return;
+   }
+   if( (int)blockIdx.x < nI0 ){
+      I0_body<R>(v, v.topo_reuse, blockIdx.x*(CB/32) + (threadIdx.x >> 5), threadIdx.x & 31);
+      return;
+   }
+   const int d = ((int)blockIdx.x - nI0)*CB + threadIdx.x;
+   if( d >= ndisk ) return;
+   if( first ) disk_begin_body<R>(v, d, 1);
+   else disk_mid_body<R>(v, d, 0.0, 1, 1);
+}
+
+/* A step's last launch: the annuli's diagnostics, and per disk the planets'
+ * update after the last substep (RK, first, advance_t as disk_mid_body) and
+ * the end of timestep(). */
 template<class R>
-__global__ void k_diag_finish(ViewT<R> v, double *Qrz, const int *ann_blk0, const int *ann_nblk){
-   int a = blockIdx.x*blockDim.x + threadIdx.x;
-   if( a < v.Nann ) diag_finish_body<R>(v, Qrz, ann_blk0, ann_nblk, a);
+__global__ void k_step_end(ViewT<R> v, int ndisk, double RK, int first, int advance_t, double *Qrz,
+                           const int *ann_blk0, const int *ann_nblk){
+   const int x = blockIdx.x*blockDim.x + threadIdx.x;
+   if( v.nq && x < v.Nann ) diag_finish_body<R>(v, Qrz, ann_blk0, ann_nblk, x);
+   if( x < ndisk ){
+      disk_mid_body<R>(v, x, RK, first, advance_t);
+      disk_end_body<R>(v, x);
+   }
 }
 
 /* ------------------------------------------------------------------ report
