@@ -191,6 +191,25 @@ static void init_planets(DiskState &S, DiskParams &D, const disco_params &p, con
    }
 }
 
+/* the block tables as the kernels read them */
+static CellBlk *upload_cell_blocks(disco_batch *b, const std::vector<int2> &blk){
+   std::vector<CellBlk> h(blk.size());
+   for( size_t i=0 ; i<blk.size() ; ++i ){
+      const int a = blk[i].x;
+      h[i] = {a, blk[i].y, b->ann_np[a], b->ann_off[a], b->ann_disk[a], b->ann_j[a], b->ann_k[a], 0};
+   }
+   return dupload(b, h);
+}
+static FaceBlk *upload_face_blocks(disco_batch *b, const std::vector<int2> &blk){
+   std::vector<FaceBlk> h(blk.size());
+   for( size_t i=0 ; i<blk.size() ; ++i ){
+      const int t = blk[i].x, A = b->tr_a[t], B = b->tr_b[t];
+      h[i] = {t, blk[i].y, b->tr_off[t], b->tr_off[t+1], A, B, b->ann_np[A], b->ann_np[B], b->ann_off[A],
+              b->ann_off[B], b->ann_disk[A], b->tr_j[t], b->tr_k[t], b->tr_dim[t], b->tr_flux[t], 0};
+   }
+   return dupload(b, h);
+}
+
 /* The radius of a track's face centres, evaluated on the host with the
  * device's operations and order (each an IEEE-rounded double operation, no
  * contraction: the sum of products as in centroid_r), and 1/(1/r) for the
@@ -737,9 +756,10 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
       b->ann_rc.push_back(host_centroid_r(rjd[j], rjd[j-1]));
    }
    v.ann_rc = dupload(b, b->ann_rc);
-   v.cblk = dupload(b, b->cblk); v.fblk = dupload(b, b->fblk); v.ublk = dupload(b, b->ublk);
-   b->d_fblk_rz = dupload(b, b->fblk_rz);
-   b->d_fblk_fl = dupload(b, b->fblk_fl);
+   v.cblk = upload_cell_blocks(b, b->cblk); v.ublk = upload_cell_blocks(b, b->ublk);
+   v.fblk = upload_face_blocks(b, b->fblk);
+   b->d_fblk_rz = upload_face_blocks(b, b->fblk_rz);
+   b->d_fblk_fl = upload_face_blocks(b, b->fblk_fl);
    v.rj = dupload(b, b->rj); v.zk = dupload(b, b->zk);
    v.dp = dupload(b, b->dparams);
    v.ds = dupload(b, dstate);

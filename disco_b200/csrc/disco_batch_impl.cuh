@@ -49,7 +49,7 @@ struct disco_batch {
    /* the same face blocks in k_faces' order (per layer, the r and z tracks of
     * each annulus together) and the blocks k_flux_t solves per direction */
    std::vector<int2> fblk_rz, fblk_fl;
-   int2 *d_fblk_rz, *d_fblk_fl;
+   FaceBlk *d_fblk_rz, *d_fblk_fl;
    int nfl_r;                           /* of fblk_fl: r-track blocks, before the z-track ones */
    std::vector<int2> ublk;              /* k_update's blocks: chunks of CB-1 cells */
    std::vector<int> ann_blk0, ann_nblk;

@@ -79,15 +79,15 @@ __device__ __forceinline__ void ct_over_runs(const ViewT<R> &v, const int *cons,
 
 template<class R>
 __global__ void __launch_bounds__(CB) k_ct_edges(ViewT<R> v){
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    if( i >= np ) return;
    const size_t N = v.Ncell;
-   int c0 = v.ann_off[a], c = c0 + i;
+   int c0 = b.c0, c = c0 + i;
    int cm = c0 + (i == 0 ? np-1 : i-1);
-   const DiskParams &P = v.dp[v.ann_disk[a]];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   const DiskParams &P = v.dp[b.disk];
+   int j = b.j, k = b.k;
    const int ne = v.ct == 2 ? 8 : 4;
    R E[8] = {0,0,0,0,0,0,0,0}, B[8] = {0,0,0,0,0,0,0,0};
    if( ct_phi_annulus(P, j, k) ){
@@ -152,15 +152,15 @@ __device__ __forceinline__ int ct_prev(const ViewT<R> &v, int a, int c){
 
 template<class R>
 __global__ void __launch_bounds__(FB) k_ct_faces(ViewT<R> v){
-   int2 b = v.fblk[blockIdx.x];
+   const FaceBlk b = v.fblk[blockIdx.x];
    int t = b.x;
-   bool zf = v.tr_dim[t] == 2;
+   bool zf = b.dim == 2;
    if( zf && v.ct != 2 ) return;
-   int f = v.tr_off[t] + b.y + threadIdx.x;
-   if( f >= v.tr_off[t+1] ) return;
+   int f = b.f0 + b.y + threadIdx.x;
+   if( f >= b.f1 ) return;
    const size_t N = v.Ncell;
-   int A = v.tr_a[t], Bn = v.tr_b[t];
-   int d = v.ann_disk[A];
+   int A = b.A, Bn = b.B;
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
    int err = 0;
    int L = v.fL[f], Rc = v.fR[f];
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(FB) k_ct_faces(ViewT<R> v){
    /* subtract_advective_B_fluxes: the owner's edge moves with its wiph; an
     * r face's edge sits at r_jph[j] (E -= h w B), a z face's at the
     * annulus centroid (E += h w B) */
-   int j = v.tr_j[t], k = v.tr_k[t];
+   int j = b.j, k = b.k;
    const double *rj = v.rj + P.rj0 + 1;
    const double *zk = v.zk + P.zk0 + 1;
    double w = v.wiph[o];
@@ -297,16 +297,16 @@ __device__ __forceinline__ R ct_ephi(const ViewT<R> &v, const DiskParams &P, int
  * minus t, the third (the diagonal annulus) a binary search. */
 template<class R>
 __global__ void __launch_bounds__(CB) k_ct_line(ViewT<R> v){
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    if( i >= np ) return;
    const size_t N = v.Ncell;
-   int c = v.ann_off[a] + i;
-   int d = v.ann_disk[a];
+   int c = b.c0 + i;
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
    if( P.Nz < 2 ) return;
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    const double *rj = v.rj + P.rj0 + 1;
    const double Pmax = P.Pmax;
    const double dt = v.ds[d].dt*v.dtfac;
@@ -422,14 +422,14 @@ __device__ __forceinline__ double ct_line_terms(const ViewT<R> &v, double S, int
  * as k_update does without CT */
 template<class R>
 __global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    if( i >= np ) return;
    const size_t N = v.Ncell;
-   int c0 = v.ann_off[a], c = c0 + i;
-   const DiskParams &P = v.dp[v.ann_disk[a]];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int c0 = b.c0, c = c0 + i;
+   const DiskParams &P = v.dp[b.disk];
+   int j = b.j, k = b.k;
    const double *X = v.fX;
    const bool z3 = v.ct == 2 && P.Nz > 1;
    /* own face f (the track's first face o) and the face before it */
@@ -510,14 +510,14 @@ __global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
  * the previous face's owner's (r and z tracks) */
 template<class R>
 __global__ void __launch_bounds__(FB) k_ct_flag(ViewT<R> v){
-   int2 b = v.fblk[blockIdx.x];
+   const FaceBlk b = v.fblk[blockIdx.x];
    int t = b.x;
-   if( v.tr_dim[t] == 2 && v.ct != 2 ) return;
-   int f = v.tr_off[t] + b.y + threadIdx.x;
-   if( f >= v.tr_off[t+1] ) return;
-   const DiskParams &P = v.dp[v.ann_disk[v.tr_a[t]]];
+   if( b.dim == 2 && v.ct != 2 ) return;
+   int f = b.f0 + b.y + threadIdx.x;
+   if( f >= b.f1 ) return;
+   const DiskParams &P = v.dp[b.disk];
    int err = 0;
-   int fm = f > v.tr_off[t] ? f-1 : v.tr_off[t+1]-1;
+   int fm = f > b.f0 ? f-1 : b.f1-1;
    int own = v.fLR[f] == 0 ? v.fL[f] : v.fR[f];
    int ownm = v.fLR[fm] == 0 ? v.fL[fm] : v.fR[fm];
    double dp = get_signed_dp(v.piph[own], v.piph[ownm], P.Pmax, &err);
@@ -615,14 +615,14 @@ __device__ void ct_cons_B(const ViewT<R> &v, const DiskParams &P, int a, int c0,
  * (prim[BZZ] dA) at its centre, into its owner's slot */
 template<int Q, int NC, class R>
 __global__ void __launch_bounds__(FB) k_ct_face_init(ViewT<R> v){
-   int2 b = v.fblk[blockIdx.x];
+   const FaceBlk b = v.fblk[blockIdx.x];
    int t = b.x;
-   bool zf = v.tr_dim[t] == 2;
+   bool zf = b.dim == 2;
    if( zf && v.ct != 2 ) return;
-   int f = v.tr_off[t] + b.y + threadIdx.x;
-   if( f >= v.tr_off[t+1] ) return;
-   const DiskParams &P = v.dp[v.ann_disk[v.tr_a[t]]];
-   int j = v.tr_j[t], k = v.tr_k[t];
+   int f = b.f0 + b.y + threadIdx.x;
+   if( f >= b.f1 ) return;
+   const DiskParams &P = v.dp[b.disk];
+   int j = b.j, k = b.k;
    const double *rj = v.rj + P.rj0 + 1;
    const double *zk = v.zk + P.zk0 + 1;
    double prim[Q];

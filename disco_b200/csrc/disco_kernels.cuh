@@ -114,6 +114,16 @@ namespace disco {
 #define MB_GR_LIGHT 6
 #endif
 
+/* A block's work and the entries of its annulus or track, in one load: read
+ * through the annulus or track index they were two more dependent loads
+ * before the block's first cell. */
+struct __align__(16) CellBlk { int x, y;          /* annulus, first cell */
+                               int np, c0, disk, j, k, pad; };
+struct __align__(16) FaceBlk { int x, y;          /* track, first face within it */
+                               int f0, f1;        /* the track's faces f0 .. f1-1 */
+                               int A, B, NA, NB, cA0, cB0;   /* its annuli, their cells */
+                               int disk, j, k, dim, flux, pad; };
+
 template<class R>
 struct ViewT {
    int Ncell, Nann, Ntr, Nf;
@@ -123,8 +133,9 @@ struct ViewT {
    const double *tr_dxL, *tr_dxR;
    const double *tr_r, *tr_irf;       /* face centre radius of the track's faces, 1/(1/r) */
    const double *ann_rc;              /* centroid radius of the annulus (get_centroid(.,.,1)) */
-   const int2 *cblk, *fblk;
-   const int2 *ublk;                  /* k_update: (annulus, first cell) of chunks of CB-1 cells */
+   const CellBlk *cblk;
+   const FaceBlk *fblk;
+   const CellBlk *ublk;               /* k_update: chunks of CB-1 cells */
    const double *rj, *zk;
    const DiskParams *dp;
    DiskState *ds;
@@ -226,11 +237,11 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid
     * side (slot t+1 = cell i0+t) */
    __shared__ R sp[Q][CB+2];
    __shared__ double sd[CB+2];
-   int2 b = v.cblk[bid];
+   const CellBlk b = v.cblk[bid];
    int a = b.x, i0 = b.y, t = threadIdx.x, i = i0 + t;
-   int np = v.ann_np[a];
+   int np = b.np;
    const int N = v.Ncell;
-   int c0 = v.ann_off[a], c = c0 + i;
+   int c0 = b.c0, c = c0 + i;
    int nact = np - i0 < CB ? np - i0 : CB;
    auto stage = [&](int slot, int cell){
 #pragma unroll
@@ -242,7 +253,7 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid
    if( t == nact-1 ) stage(nact+1, c0 + (i0+nact == np ? 0 : i0+nact));
    __syncthreads();
    if( t >= nact ) return;
-   int d = v.ann_disk[a];
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
 
    R pC[Q], pL[Q], pR[Q];
@@ -254,7 +265,7 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid
       double w = 0.0;
       if constexpr ( GR ){          /* get_omega of grmhd2, grmhd2.c:64-86 (set_wcell's x) */
          if( P.mesh_motion ){
-            int j = v.ann_j[a], k = v.ann_k[a];
+            int j = b.j, k = b.k;
             const double *rj = v.rj + P.rj0 + 1, *zk = v.zk + P.zk0 + 1;
             double x[3] = {centroid_r(rj[j], rj[j-1]), 0.0, centroid_z(zk[k], zk[k-1])};
             double pc[Q], pr[Q];
@@ -267,7 +278,7 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid
          if( P.mesh_motion ) w = .5*((double)pC[UPP] + (double)pR[UPP]);   /* get_omega = prim[UPP] */
       }
       if( P.mesh_motion == 4 ){
-         int j = v.ann_j[a];
+         int j = b.j;
          const double *rj = v.rj + P.rj0 + 1;
          w = mesh_om(P, centroid_r(rj[j], rj[j-1]));
       }
@@ -476,16 +487,16 @@ __device__ __forceinline__ int gallop_lb(int lo, int hi, int g, Pr p){
  * the two cells' scattered states was measured 5x slower than storing. */
 template<int Q, class R>
 __device__ __forceinline__ void faces_body(const ViewT<R> &v, int with_slopes, int topo_reuse, int bid){
-   int2 b = v.fblk[bid];
+   const FaceBlk b = v.fblk[bid];
    int t = b.x, dd = b.y + threadIdx.x;
-   int A = v.tr_a[t], B = v.tr_b[t];
-   int NA = v.ann_np[A], NB = v.ann_np[B];
+   int A = b.A, B = b.B;
+   int NA = b.NA, NB = b.NB;
    if( dd >= NA + NB ) return;
    const int N = v.Ncell;
-   int f = v.tr_off[t] + dd;
-   int cA0 = v.ann_off[A], cB0 = v.ann_off[B];
+   int f = b.f0 + dd;
+   int cA0 = b.cA0, cB0 = b.cB0;
    int IA = v.I0[A], IB = v.I0[B];
-   const DiskParams &P = v.dp[v.ann_disk[A]];
+   const DiskParams &P = v.dp[b.disk];
    double Pmax = P.Pmax;
    int err = 0;
 
@@ -535,13 +546,13 @@ __device__ __forceinline__ void faces_body(const ViewT<R> &v, int with_slopes, i
    double xp1 = LR == 0 ? pL : pR;
    double xm1 = LR_back == 0 ? pL-dL : pR-dR;
 
-   int j = v.tr_j[t], k = v.tr_k[t];
+   int j = b.j, k = b.k;
    const double *rj = v.rj + P.rj0 + 1;
    const double *zk = v.zk + P.zk0 + 1;
    double dp = get_dp(xp1, xm1, Pmax, &err);
    double phic = get_dp(xp1, .5*dp, Pmax, &err);
    double dA;
-   if( v.tr_dim[t] == 1 ){
+   if( b.dim == 1 ){
       double r = .5*(rj[j]+rj[j]);
       double dz = zk[k]-zk[k-1];
       dA = r*dp*dz;                                       /* get_dA(.,.,1) */
@@ -553,7 +564,7 @@ __device__ __forceinline__ void faces_body(const ViewT<R> &v, int with_slopes, i
 
    v.fL[f] = cL; v.fR[f] = cR; v.fLR[f] = (unsigned char)LR;
    v.fphic[f] = phic; v.fdA[f] = dA; v.fdp[f] = dp;
-   if( v.tr_dim[t] == 1 ){ if( LR == 0 ) v.consL[cL] = f; else v.consR[cR] = f; }
+   if( b.dim == 1 ){ if( LR == 0 ) v.consL[cL] = f; else v.consR[cR] = f; }
    else                  { if( LR == 0 ) v.consZL[cL] = f; else v.consZR[cR] = f; }
 
    if( with_slopes ){
@@ -606,17 +617,17 @@ __device__ __forceinline__ Runs cell_runs(const ViewT<R> &v, const int *cons, in
  * every face's limiter. */
 template<int Q, int DIM, class R>
 __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
-   int2 b = v.cblk[bid];
+   const CellBlk b = v.cblk[bid];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    if( i >= np ) return;
    const int N = v.Ncell;
-   int c0 = v.ann_off[a], c = c0 + i;
-   int d = v.ann_disk[a];
+   int c0 = b.c0, c = c0 + i;
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
    if( DIM == 2 && P.Nz == 1 ) return;
    R *grad = DIM == 1 ? v.gradr : v.gradz;
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    int Nr = P.Nr, Nz = P.Nz;
    int I0 = v.I0[a];
    R g[Q];
@@ -804,15 +815,15 @@ __device__ __forceinline__ double2 visc_source_cell(const ViewT<R> &v, const Dis
  * (addFace, faces_alt.c:10-16). */
 template<int Q, int NC, int DIM, class R, bool VISC = false, bool GR = false>
 __device__ __forceinline__ void flux_body(const ViewT<R> &v, double dtfac, int bid){
-   int2 b = v.fblk[bid];
+   const FaceBlk b = v.fblk[bid];
    int t = b.x;
-   if( v.tr_dim[t] != DIM || !v.tr_flux[t] ) return;
+   if( b.dim != DIM || !b.flux ) return;
    int dd = b.y + threadIdx.x;
-   int f = v.tr_off[t] + dd;
-   if( f >= v.tr_off[t+1] ) return;
+   int f = b.f0 + dd;
+   if( f >= b.f1 ) return;
    const int N = v.Ncell;
    int cL = v.fL[f], cR = v.fR[f];
-   int d = v.ann_disk[v.tr_a[t]];
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
    int err = 0;
    double dt = v.ds[d].dt*dtfac;
@@ -841,7 +852,7 @@ __device__ __forceinline__ void flux_body(const ViewT<R> &v, double dtfac, int b
    R G[Q];
    if constexpr ( GR ){              /* grmhd2 + HLL at the face centre (addFace, faces_alt.c:10-16) */
       const double *zk = v.zk + P.zk0 + 1;
-      int k = v.tr_k[t];
+      int k = b.k;
       double x[3] = {r, phi, DIM == 1 ? 0.5*(zk[k]+zk[k-1]) : 0.5*(zk[k]+zk[k])};
       const double n[3] = {DIM == 1 ? 1.0 : 0.0, 0.0, DIM == 2 ? 1.0 : 0.0};
       double pl[Q], pr[Q], g[Q];
@@ -991,15 +1002,15 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
     * chunk's last). */
    __shared__ R sG[Q][CB];
    __shared__ R sW[Q][CB+1];      /* sW[.][s]: left-edge state of cell i0+s-1 */
-   int2 b = v.ublk[bid];
+   const CellBlk b = v.ublk[bid];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    const int N = v.Ncell;
-   int c0 = v.ann_off[a], c = c0 + i;
+   int c0 = b.c0, c = c0 + i;
    int cprev = c0 + (i == 0 ? np-1 : i-1);
-   int d = v.ann_disk[a];
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    bool real = j >= P.NgRa && j < P.Nr - P.NgRb && k >= P.NgZa && k < P.Nz - P.NgZb;
    const double *rj = v.rj + P.rj0 + 1;
    const double *zk = v.zk + P.zk0 + 1;
@@ -1309,13 +1320,13 @@ __device__ __forceinline__ int diag_slot(int m){ return m == NQD ? DIAG_VOL : m;
 template<int Q, class R, int NQD>
 __global__ void __launch_bounds__(CB) k_diag_part(ViewT<R> v){
    __shared__ double s_red[CB/32][NQD+1];
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    const int N = v.Ncell;
-   int d = v.ann_disk[a];
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    const double *rj = v.rj + P.rj0 + 1;
    const double *zk = v.zk + P.zk0 + 1;
    double dq[NQD+1];
@@ -1323,7 +1334,7 @@ __global__ void __launch_bounds__(CB) k_diag_part(ViewT<R> v){
    for( int m=0 ; m<=NQD ; ++m ) dq[m] = 0.0;
    int err = 0;
    if( i < np ){
-      int c = v.ann_off[a] + i;
+      int c = b.c0 + i;
       double prim[Q];
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[q*N + c];
@@ -1649,15 +1660,15 @@ __device__ __forceinline__ void c2p_tail(const ViewT<R> &v, const DiskParams &P,
 template<int Q, int NC, class R, int NQD = 5, bool VISC = false, bool GR = false>
 __device__ __forceinline__ void c2p_body(const ViewT<R> &v, int last, int bc, int diag, int move_c2p,
                                          int topo_set, int bid){
-   int2 b = v.cblk[bid];
+   const CellBlk b = v.cblk[bid];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    bool active = i < np;
    const int N = v.Ncell;
-   int c0 = v.ann_off[a], c = c0 + (active ? i : 0);
-   int d = v.ann_disk[a];
+   int c0 = b.c0, c = c0 + (active ? i : 0);
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    bool real = j >= P.NgRa && j < P.Nr - P.NgRb && k >= P.NgZa && k < P.Nz - P.NgZb;
    int err = 0;
    double cons[Q];
@@ -2066,14 +2077,14 @@ enum { RP_PSIR, RP_PSII, RP_L1ISEN, RP_L1RHO, RP_L1P, RP_L1B, RP_BR2, RP_BRBP, R
 template<int Q, int NC, class R>
 __global__ void __launch_bounds__(CB) k_report_part(ViewT<R> v, double *part){
    __shared__ double s_red[CB/32][RP_N];
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    const int N = v.Ncell;
-   int d = v.ann_disk[a];
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
    const DiskState &S = v.ds[d];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    bool real = j >= P.NgRa && j < P.Nr - P.NgRb && k >= P.NgZa && k < P.Nz - P.NgZb;
    double x[RP_N];
 #pragma unroll
@@ -2081,7 +2092,7 @@ __global__ void __launch_bounds__(CB) k_report_part(ViewT<R> v, double *part){
    x[RP_RHOMIN] = HUGE_VAL;
    int err = 0;
    if( real && i < np ){
-      int c = v.ann_off[a] + i;
+      int c = b.c0 + i;
       const double *rj = v.rj + P.rj0 + 1;
       const double *zk = v.zk + P.zk0 + 1;
       double phip = v.piph[c], dphi = v.dphi[c];
@@ -2197,15 +2208,15 @@ __global__ void k_report_finish(ViewT<R> v, const double *part, const int *ann_b
  * cells (FP64); then main.c's boundary_trans for ghosts. */
 template<int Q, int NC, class R>
 __global__ void __launch_bounds__(CB) k_setup(ViewT<R> v, int bc){
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    if( i >= np ) return;
    const int N = v.Ncell;
-   int c = v.ann_off[a] + i;
-   int d = v.ann_disk[a];
+   int c = b.c0 + i;
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    const double *rj = v.rj + P.rj0 + 1;
    const double *zk = v.zk + P.zk0 + 1;
    bool real = j >= P.NgRa && j < P.Nr - P.NgRb && k >= P.NgZa && k < P.Nz - P.NgZb;
@@ -2285,15 +2296,15 @@ __global__ void __launch_bounds__(CB) k_setup(ViewT<R> v, int bc){
  * nothing reads them). */
 template<int Q, int NC, class R>
 __global__ void __launch_bounds__(CB) k_restart(ViewT<R> v, int bc){
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    if( i >= np ) return;
    const int N = v.Ncell;
-   int c0 = v.ann_off[a], c = c0 + i;
-   int d = v.ann_disk[a];
+   int c0 = b.c0, c = c0 + i;
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    const double *rj = v.rj + P.rj0 + 1;
    const double *zk = v.zk + P.zk0 + 1;
    bool real = j >= P.NgRa && j < P.Nr - P.NgRb && k >= P.NgZa && k < P.Nz - P.NgZb;
@@ -2356,14 +2367,14 @@ __global__ void __launch_bounds__(CB) k_restart(ViewT<R> v, int bc){
 /* prim2cons on real cells for an upload without cons (domain.c:349). */
 template<int Q, int NC, class R>
 __global__ void __launch_bounds__(CB) k_prim2cons(ViewT<R> v){
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    if( i >= np ) return;
    const int N = v.Ncell;
-   int c = v.ann_off[a] + i;
-   const DiskParams &P = v.dp[v.ann_disk[a]];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int c = b.c0 + i;
+   const DiskParams &P = v.dp[b.disk];
+   int j = b.j, k = b.k;
    const double *rj = v.rj + P.rj0 + 1;
    const double *zk = v.zk + P.zk0 + 1;
    int err = 0;
@@ -2394,20 +2405,20 @@ __global__ void __launch_bounds__(CB) k_prim2cons(ViewT<R> v){
 /* set_wcell alone (setupCells' last call, domain.c:385). */
 template<int Q, class R>
 __global__ void __launch_bounds__(CB) k_wcell(ViewT<R> v){
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    if( i >= np ) return;
    const int N = v.Ncell;
-   int c0 = v.ann_off[a], c = c0 + i;
+   int c0 = b.c0, c = c0 + i;
    int cp = c0 + (i+1 == np ? 0 : i+1);
-   const DiskParams &P = v.dp[v.ann_disk[a]];
+   const DiskParams &P = v.dp[b.disk];
    double w = 0.0;
    bool gr = false;
    if constexpr ( Q == 9 && sizeof(R) == sizeof(double) ) gr = P.gr;
    if( gr ){                        /* set_wcell with grmhd2's get_omega */
       if( P.mesh_motion ){
-         int j = v.ann_j[a], k = v.ann_k[a];
+         int j = b.j, k = b.k;
          const double *rj = v.rj + P.rj0 + 1, *zk = v.zk + P.zk0 + 1;
          double x[3] = {centroid_r(rj[j], rj[j-1]), 0.0, centroid_z(zk[k], zk[k-1])};
          double pc[Q], pr[Q];
@@ -2416,7 +2427,7 @@ __global__ void __launch_bounds__(CB) k_wcell(ViewT<R> v){
       }
    }else if( P.mesh_motion ) w = .5*((double)v.prim[UPP*N + c] + (double)v.prim[UPP*N + cp]);
    if( P.mesh_motion == 4 ){
-      int j = v.ann_j[a];
+      int j = b.j;
       const double *rj = v.rj + P.rj0 + 1;
       w = mesh_om(P, centroid_r(rj[j], rj[j-1]));
    }
@@ -2427,14 +2438,14 @@ __global__ void __launch_bounds__(CB) k_wcell(ViewT<R> v){
 template<int Q, int NC, class R>
 __global__ void __launch_bounds__(CB) k_mindt(ViewT<R> v){
    __shared__ unsigned long long s_dt[CB/32];
-   int2 b = v.cblk[blockIdx.x];
+   const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
-   int np = v.ann_np[a];
+   int np = b.np;
    const int N = v.Ncell;
-   int c0 = v.ann_off[a];
-   int d = v.ann_disk[a];
+   int c0 = b.c0;
+   int d = b.disk;
    const DiskParams &P = v.dp[d];
-   int j = v.ann_j[a], k = v.ann_k[a];
+   int j = b.j, k = b.k;
    bool real = j >= P.NgRa && j < P.Nr - P.NgRb && k >= P.NgZa && k < P.Nz - P.NgZb;
    double dtc = 1.0e300;
    int err = 0;
