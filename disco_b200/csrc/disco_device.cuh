@@ -819,8 +819,17 @@ __device__ __forceinline__ void planetary_force_sc(int grav2D, const Planet &pl,
    else if( grav2D == 2 ){ rp = r; cpp = cosp; spp = sinp; z = 1.0; }
    double dx = r*cosp-rp*cpp;
    double dy = r*sinp-rp*spp;
-   double script_r = sqrt(dx*dx+dy*dy+z*z);
    double script_r_perp = sqrt(dx*dx+dy*dy);
+   /* at z = 0 (2D disks, cylindrical gravity) the distance is the one in the
+    * plane, and its two ratios are 1 and z, bit for bit: a square root and
+    * two divisions of the eight saved in every cell for every planet */
+   const bool flat = z == 0.0 && script_r_perp > 0.0 && script_r_perp < 1.0e300;
+   double script_r = script_r_perp, sint = 1.0, cost = z;
+   if( !flat ){
+      script_r = sqrt(dx*dx+dy*dy+z*z);
+      sint = script_r_perp/script_r;
+      cost = z/script_r;
+   }
    double f1 = -fgrav( pl.M , script_r , pl.eps , pl.type );
    double cosa = dx/script_r_perp;
    double sina = dy/script_r_perp;
@@ -831,8 +840,6 @@ __device__ __forceinline__ void planetary_force_sc(int grav2D, const Planet &pl,
       sinap = sina*cpp-cosa*spp;
    }
    if( script_r_perp <= 0.0 ){ cosap = 0.0; sinap = 0.0; }
-   double sint = script_r_perp/script_r;
-   double cost = z/script_r;
    *fr = cosap*f1*sint;
    *fp = sinap*f1*sint;
    *fz = f1*cost;

@@ -206,6 +206,12 @@ struct ViewT {
    double *lineX;
 };
 
+/* start the line holding *p on its way to L2 (no register waits for it) */
+template<class T>
+__device__ __forceinline__ void prefetch_l2(const T *p){
+   asm volatile("prefetch.global.L2 [%0];" :: "l"(p));
+}
+
 template<class R>
 __device__ __forceinline__ void raise_err(const ViewT<R> &v, int e){
    if( e ) atomicOr(v.err, e);
@@ -1024,6 +1030,17 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
          int kmin = P.NgZa == 0 ? 0 : P.NgZa-1, kmax = P.NgZb == 0 ? P.Nz : P.Nz-P.NgZb+1;
          ctE = j >= jmin && j < jmax && k >= kmin && k < kmax;
       }
+   }
+   if( real && threadIdx.x < CB-1 && i < np ){
+      /* what the gather reads after the phi faces, on its way to L2 meanwhile */
+#pragma unroll
+      for( int q=0 ; q<Q ; ++q ){
+         prefetch_l2(v.cons + (size_t)q*N + c);
+         if( !first ) prefetch_l2(v.RKcons + (size_t)q*N + c);
+         if constexpr ( sizeof(R) != sizeof(double) ) prefetch_l2(v.ccarry + (size_t)q*N + c);
+      }
+      prefetch_l2(v.consL + c); prefetch_l2(v.consR + c);
+      if( P.Nz > 1 ){ prefetch_l2(v.consZL + c); prefetch_l2(v.consZR + c); }
    }
    if( real || ctE ){               /* uniform over the block: one annulus */
       double dA = (rj[j]-rj[j-1])*(zk[k]-zk[k-1]);       /* get_dA(.,.,0) */
