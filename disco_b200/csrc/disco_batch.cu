@@ -910,6 +910,7 @@ extern "C" void disco_batch_destroy(disco_batch *b){
    if( b->d_stage ) cudaFree(b->d_stage);
    if( b->d_rpart ) cudaFree(b->d_rpart);
    if( b->d_rout ) cudaFree(b->d_rout);
+   if( b->h_ds ) cudaFreeHost(b->h_ds);
    delete b;
 }
 
@@ -931,7 +932,10 @@ static cudaError_t xfer(const disco_batch *b, void *dst, const void *src, size_t
 
 /* cell-major FP64 (Q per cell) host <-> SoA device of element type T: one
  * contiguous copy through a device staging array (DMA at full speed when the
- * host buffer is pinned), transposed on the device, one thread per cell. */
+ * host buffer is pinned), transposed on the device, one thread per cell.
+ * The copies of a call are queued on the batch's stream one after another
+ * (the staging array is free again when the stream reaches the next); the
+ * caller of upload_q / download_q synchronises once, before it returns. */
 template<class T>
 __global__ void k_aos_to_soa(const double *src, T *dst, size_t N, int Q){
    size_t c = blockIdx.x*(size_t)blockDim.x + threadIdx.x;
@@ -962,7 +966,6 @@ static int upload_q(disco_batch *b, T *dst, const double *src, int Q = 0){
    CK(cudaMemcpyAsync(b->d_stage, src, (size_t)Q*N*sizeof(double), cudaMemcpyHostToDevice, b->stream));
    k_aos_to_soa<T><<<nblk(N, 256), 256, 0, b->stream>>>(b->d_stage, dst, N, Q);
    CK(cudaGetLastError());
-   CK(cudaStreamSynchronize(b->stream));
    return DISCO_OK;
 }
 template<class T>
@@ -973,7 +976,7 @@ static int download_q(disco_batch *b, double *dst, const T *src, int Q = 0){
    if( s ) return s;
    k_soa_to_aos<T><<<nblk(N, 256), 256, 0, b->stream>>>(src, b->d_stage, N, Q);
    CK(cudaGetLastError());
-   CK(xfer(b, dst, b->d_stage, (size_t)Q*N*sizeof(double), cudaMemcpyDeviceToHost));
+   CK(cudaMemcpyAsync(dst, b->d_stage, (size_t)Q*N*sizeof(double), cudaMemcpyDeviceToHost, b->stream));
    return DISCO_OK;
 }
 /* an R-typed cell array of the batch (prim, gradp, gradr) */
@@ -1003,9 +1006,12 @@ extern "C" int disco_batch_set_cells(disco_batch *b, const double *prim, const d
          CK(cudaMemsetAsync(b->vd.Phi, 0, (size_t)b->nfs*N*sizeof(double), b->stream));
       }
    }
-   CK(xfer(b, b->vd.piph, piph, N*sizeof(double), cudaMemcpyHostToDevice));
-   CK(xfer(b, b->vd.dphi, dphi, N*sizeof(double), cudaMemcpyHostToDevice));
-   if( wiph ) CK(xfer(b, b->vd.wiph, wiph, N*sizeof(double), cudaMemcpyHostToDevice));
+   auto up = [&](double *dev, const double *src){
+      return cudaMemcpyAsync(dev, src, N*sizeof(double), cudaMemcpyHostToDevice, b->stream);
+   };
+   CK(up(b->vd.piph, piph));
+   CK(up(b->vd.dphi, dphi));
+   if( wiph ) CK(up(b->vd.wiph, wiph));
    if( b->vd.ccarry ) CK(cudaMemsetAsync(b->vd.ccarry, 0, (size_t)b->Q*N*sizeof(float), b->stream));
    b->topo_known = 0;
    CK(cudaMemsetAsync(b->vd.topo, 0, sizeof(int), b->stream));      /* new piph: faces stale */
@@ -1024,15 +1030,18 @@ extern "C" int disco_batch_get_cells(disco_batch *b, double *prim, double *cons,
                                      double *piph, double *dphi, double *wiph, double *Phi){
    if( !b ) return DISCO_ERR_ARG;
    CK(cudaSetDevice(b->device));
-   CK(cudaStreamSynchronize(b->stream));
    size_t N = b->ncell;
    int s;
    if( Phi && b->ct && (s = download_q<double>(b, Phi, b->vd.Phi, b->nfs)) ) return s;
    if( prim && (s = download_r(b, prim, b->vd.prim)) ) return s;
    if( cons && (s = download_q<double>(b, cons, b->vd.cons)) ) return s;
-   if( piph ) CK(xfer(b, piph, b->vd.piph, N*sizeof(double), cudaMemcpyDeviceToHost));
-   if( dphi ) CK(xfer(b, dphi, b->vd.dphi, N*sizeof(double), cudaMemcpyDeviceToHost));
-   if( wiph ) CK(xfer(b, wiph, b->vd.wiph, N*sizeof(double), cudaMemcpyDeviceToHost));
+   auto down = [&](double *dst, const double *dev){
+      return cudaMemcpyAsync(dst, dev, N*sizeof(double), cudaMemcpyDeviceToHost, b->stream);
+   };
+   if( piph ) CK(down(piph, b->vd.piph));
+   if( dphi ) CK(down(dphi, b->vd.dphi));
+   if( wiph ) CK(down(wiph, b->vd.wiph));
+   CK(cudaStreamSynchronize(b->stream));
    return DISCO_OK;
 }
 
@@ -1099,13 +1108,20 @@ extern "C" int disco_batch_mindt(disco_batch *b, double *dt){
    CK(cudaSetDevice(b->device));
    int s = launch_mindt(b);
    if( s ) return s;
-   CK(cudaStreamSynchronize(b->stream));
-   if( dt ){
-      std::vector<DiskState> st(b->ndisk);
-      CK(xfer(b, st.data(), b->vd.ds, sizeof(DiskState)*b->ndisk, cudaMemcpyDeviceToHost));
-      for( int d=0 ; d<b->ndisk ; ++d ) dt[d] = st[d].dt_next;
+   /* the disks' states and the error word in one wait, through a pinned
+    * mirror: a host dt loop makes this round trip every step */
+   if( !b->h_ds ){
+      if( cudaMallocHost((void **)&b->h_ds, sizeof(DiskState)*b->ndisk + sizeof(int)) != cudaSuccess ){
+         b->h_ds = NULL;
+         return DISCO_ERR_CUDA;
+      }
    }
-   return read_err(b);
+   int *h_err = (int *)(b->h_ds + b->ndisk);
+   CK(cudaMemcpyAsync(b->h_ds, b->vd.ds, sizeof(DiskState)*b->ndisk, cudaMemcpyDeviceToHost, b->stream));
+   CK(cudaMemcpyAsync(h_err, b->d_err, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+   CK(cudaStreamSynchronize(b->stream));
+   if( dt ) for( int d=0 ; d<b->ndisk ; ++d ) dt[d] = b->h_ds[d].dt_next;
+   return *h_err ? read_err(b) : DISCO_OK;
 }
 
 static void launch_step(disco_batch *b, int use_next){
@@ -1113,15 +1129,23 @@ static void launch_step(disco_batch *b, int use_next){
    else launch_step_t(b, b->vd, use_next);
 }
 
+/* the dt of up to N disks, a kernel argument */
+struct DtChunk { enum { N = 64 }; int n; double dt[N]; };
+__global__ void k_set_dt(DiskState *ds, DtChunk ch){
+   if( (int)threadIdx.x < ch.n ) ds[threadIdx.x].dt_next = ch.dt[threadIdx.x];
+}
+
 extern "C" int disco_batch_timestep(disco_batch *b, const double *dt){
    if( !b ) return DISCO_ERR_ARG;
    if( !b->have_cells ) return DISCO_ERR_STATE;
    CK(cudaSetDevice(b->device));
-   if( dt ){
-      std::vector<DiskState> st(b->ndisk);
-      CK(xfer(b, st.data(), b->vd.ds, sizeof(DiskState)*b->ndisk, cudaMemcpyDeviceToHost));
-      for( int d=0 ; d<b->ndisk ; ++d ) st[d].dt_next = dt[d];
-      CK(xfer(b, b->vd.ds, st.data(), sizeof(DiskState)*b->ndisk, cudaMemcpyHostToDevice));
+   if( dt ){                        /* by value with the launch: no copy, no wait */
+      for( int d0=0 ; d0<b->ndisk ; d0+=DtChunk::N ){
+         DtChunk ch;
+         ch.n = b->ndisk - d0 < DtChunk::N ? b->ndisk - d0 : DtChunk::N;
+         memcpy(ch.dt, dt + d0, sizeof(double)*ch.n);
+         k_set_dt<<<1, DtChunk::N, 0, b->stream>>>(b->vd.ds + d0, ch);
+      }
    }
    launch_step(b, 1);
    CK(cudaGetLastError());
@@ -1357,11 +1381,12 @@ extern "C" int disco_batch_last_error(disco_batch *b){
 extern "C" int disco_batch_debug_get(disco_batch *b, int which, double *out){
    if( !b || !out ) return DISCO_ERR_ARG;
    CK(cudaSetDevice(b->device));
-   CK(cudaStreamSynchronize(b->stream));
-   if( which == 0 ) return download_r(b, out, b->vd.gradp);
-   if( which == 1 ) return download_r(b, out, b->vd.gradr);
-   if( which == 2 ) return download_q<double>(b, out, b->vd.RKcons);
-   return DISCO_ERR_ARG;
+   int s = DISCO_ERR_ARG;
+   if( which == 0 ) s = download_r(b, out, b->vd.gradp);
+   if( which == 1 ) s = download_r(b, out, b->vd.gradr);
+   if( which == 2 ) s = download_q<double>(b, out, b->vd.RKcons);
+   if( s == DISCO_OK ) CK(cudaStreamSynchronize(b->stream));
+   return s;
 }
 
 extern "C" int disco_batch_set_stream(disco_batch *b, void *stream){
