@@ -806,6 +806,7 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
       v.pE = ralloc(N); v.pB = ralloc(N);
       v.fEt = ralloc(face); v.fBt = ralloc(face);
       v.fX = dalloc<double>(b, face);
+      v.fPhi = dalloc<double>(b, face);
       v.fFlip = dalloc<unsigned char>(b, face);
       if( ct == 2 ){
          v.pEr = ralloc(N); v.pBz = ralloc(N);
@@ -825,7 +826,7 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
             b->d_zpole = dupload(b, b->zpole);
          }
          if( b->any_3d ){
-            v.rk = dalloc<int>(b, 4*N);
+            v.frk = dalloc<int>(b, 2*(size_t)face);
             v.lineX = dalloc<double>(b, (size_t)b->line_ne);
             v.line_off = dupload(b, b->line_off);
          }

@@ -287,132 +287,157 @@ __device__ __forceinline__ R ct_ephi(const ViewT<R> &v, const DiskParams &P, int
    return v.tr_flux[t] ? v.fEphi[f] : R(0.0);
 }
 
-/* make_edge_adjust, one thread per (cell, list): the line (jl, kl) is the
- * r_jph[jl], z_kph[kl] edge; its lists are the annuli (jl,kl) [c],
- * (jl+1,kl) [cR], (jl,kl+1) [cU], (jl+1,kl+1) [cUR], each from its I0, and
- * the reference merges them by repeated get_which4, ties to the lower list
- * index.  A cell of list m at position t is consumed at step
- * e = t + (cells of each other list before it): two of those counts are the
- * cell's position in the face list of the track it shares with that list
- * minus t, the third (the diagonal annulus) a binary search. */
+/* make_edge_adjust, one thread per cell, which is list M (0..3) of the four
+ * lines it borders: the line (jl, kl) is the r_jph[jl], z_kph[kl] edge; its
+ * lists are the annuli (jl,kl) [c], (jl+1,kl) [cR], (jl,kl+1) [cU],
+ * (jl+1,kl+1) [cUR], each from its I0, and the reference merges them by
+ * repeated get_which4, ties to the lower list index.  A cell of list M at
+ * position t is consumed at step e = t + (cells of each other list before
+ * it): two of those counts are the cell's position in the face list of the
+ * track it shares with that list minus t, the third (the diagonal annulus) a
+ * binary search.
+ *
+ * The step's rank is stored at the two faces the cell ends there (frk: for
+ * an r face the line below it in slot 0, above it in slot 1; for a z face
+ * the line inside / outside it), where k_ct_update reads it beside its
+ * neighbours.  Instruction-bound: the lists are numbered at compile time
+ * (indexed at run time, the counts and cells lay in local memory and each
+ * step branched four ways on the list consumed), and the 3 x 3 annuli around
+ * the block are read once, into shared memory. */
+struct LineAnn { int off, np, I0; };
+
+template<int M, class R>
+__device__ __forceinline__ void ct_line_step(const ViewT<R> &v, const DiskParams &P, const LineAnn (*A)[3],
+                                             const int *f4, const int *o4, int c, int j, int k, int t, int np,
+                                             double ux, double dt, int *err){
+   const int jl = j - (M & 1), kl = k - (M >> 1);
+   if( jl < 0 || jl > P.Nr-2 || kl < 0 || kl > P.Nz-2 ) return;
+   const double Pmax = P.Pmax;
+   /* the cell's r and z face of this line (0 inner r, 1 outer r, 2 lower z,
+    * 3 upper z), and the counts their lists give */
+   constexpr int sr = (M & 1) ? 0 : 1, sz = (M >> 1) ? 2 : 3;
+   const int fr = f4[sr], fz = f4[sz];
+   /* list n's annulus, relative to the cell's */
+   auto ann = [&](int n) -> const LineAnn & { return A[1 + (n >> 1) - (M >> 1)][1 + (n & 1) - (M & 1)]; };
+   int cnt[4];
+   cnt[M] = t;
+   cnt[M ^ 1] = fr - o4[sr] - t;
+   cnt[M ^ 2] = fz - o4[sz] - t;
+   {                                /* diagonal: cells of list n before this one */
+      constexpr int n = M ^ 3;
+      const LineAnn a = ann(n);
+      /* both lists unrolled from I0: the count is near t nn / np */
+      cnt[n] = gallop_lb(0, a.np, __float2int_rz(__fdividef((float)t*(float)a.np, (float)np)), [&](int mid){
+         int s = a.I0 + mid; if( s >= a.np ) s -= a.np;
+         double uy = v.piph[a.off + s];
+         return !(n < M ? uy <= ux : uy < ux);
+      });
+   }
+   const int e = cnt[0] + cnt[1] + cnt[2] + cnt[3];
+   const int line = P.ln0 + jl + (P.Nr-1)*kl;
+   const int l0 = v.line_off[line];
+   if( e < 0 || e >= v.line_off[line+1] - l0 ){ *err |= ERRF_INTERNAL; return; }
+   const size_t Nf = v.Nf;
+   v.frk[(M >> 1) ? fr : Nf + fr] = e;
+   v.frk[(M & 1) ? fz : Nf + fz] = e;
+   /* the reference's state at step e */
+   int cur[4];
+   bool bad = false;
+#pragma unroll
+   for( int n=0 ; n<4 ; ++n ){
+      if( n == M ){ cur[n] = c; continue; }
+      const LineAnn a = ann(n);
+      int s = a.I0 + cnt[n];                 /* I0 < np, 0 <= cnt <= np */
+      if( s >= a.np ) s -= a.np;
+      if( s < 0 || s >= a.np ){ bad = true; s = 0; }
+      cur[n] = a.off + s;
+   }
+   if( bad ){ *err |= ERRF_INTERNAL; return; }
+   double xp[4], xm[4];
+#pragma unroll
+   for( int n=0 ; n<4 ; ++n ){ xp[n] = n == M ? ux : v.piph[cur[n]]; xm[n] = xp[n] - v.dphi[cur[n]]; }
+   int LR_alt = 0, UD_alt = 0;
+   const int w4 = ct_which4(xp[0], xp[1], xp[2], xp[3], &LR_alt, &UD_alt, 0, Pmax, err);
+   const int w4b = ct_which4(xm[0], xm[1], xm[2], xm[3], NULL, NULL, 1, Pmax, err);
+   if( w4 != M ) *err |= ERRF_INTERNAL;
+   /* E_phi of the cells' owned faces: c [3],[1]; cR [3],[0]; cU [1],[2];
+    * cUR [0],[2]: the cell's own two, and one of the other row's and of the
+    * other column's each */
+   auto eph = [&](int n, int s){ return ct_ephi(v, P, cur[n], jl + (n & 1), kl + (n >> 1), s); };
+   auto own = [&](int s, int f){
+      const int tr = s <= 1 ? P.trr0 + jl + (P.Nr-1)*k : P.trz0 + j + P.Nr*kl;
+      return v.tr_flux[tr] ? v.fEphi[f] : R(0.0);
+   };
+   const R q4 = R(.25);
+   R E = q4*( own(sz, fz) + own(sr, fr) );
+   if( M < 2 ){ if( LR_alt == 0 ) E += q4*eph(2,1); else E += q4*eph(3,0); }
+   else       { if( LR_alt == 0 ) E += q4*eph(0,1); else E += q4*eph(1,0); }
+   if( (M & 1) == 0 ){ if( UD_alt == 0 ) E += q4*eph(1,3); else E += q4*eph(3,2); }
+   else              { if( UD_alt == 0 ) E += q4*eph(0,3); else E += q4*eph(2,2); }
+   const double xmb = w4b == 0 ? xm[0] : w4b == 1 ? xm[1] : w4b == 2 ? xm[2] : xm[3];
+   const double *rj = v.rj + P.rj0 + 1;
+   double dl = (.5*(rj[jl]+rj[jl]))*get_dp(ux, xmb, Pmax, err);     /* get_dL(.,.,0) */
+   v.lineX[l0 + e] = (double)E*dl*dt;
+}
+
 template<class R>
 __global__ void __launch_bounds__(CB) k_ct_line(ViewT<R> v){
+   __shared__ LineAnn A[3][3];
+   __shared__ int s_o[4];
    const CellBlk b = v.cblk[blockIdx.x];
-   int a = b.x, i = b.y + threadIdx.x;
-   int np = b.np;
-   if( i >= np ) return;
-   const size_t N = v.Ncell;
-   int c = b.c0 + i;
-   int d = b.disk;
-   const DiskParams &P = v.dp[d];
+   const int i = b.y + threadIdx.x, np = b.np, j = b.j, k = b.k;
+   const DiskParams &P = v.dp[b.disk];
    if( P.Nz < 2 ) return;
-   int j = b.j, k = b.k;
-   const double *rj = v.rj + P.rj0 + 1;
-   const double Pmax = P.Pmax;
-   const double dt = v.ds[d].dt*v.dtfac;
-   int err = 0;
-   int t = i - v.I0[a];
-   if( t < 0 ) t += np;
-   double ux = v.piph[c];
-   for( int m=0 ; m<4 ; ++m ){
-      int jl = j - (m & 1), kl = k - (m >> 1);
-      if( jl < 0 || jl > P.Nr-2 || kl < 0 || kl > P.Nz-2 ) continue;
-      int an[4], cnt[4];
-      for( int n=0 ; n<4 ; ++n ) an[n] = P.ann0 + (jl + (n & 1)) + P.Nr*(kl + (n >> 1));
-      cnt[m] = t;
-      for( int n=0 ; n<4 ; ++n ){
-         if( n == m ) continue;
-         int x = n ^ m;
-         if( x == 1 ){                /* same layer: the r-track of that layer */
-            int tr = P.trr0 + jl + (P.Nr-1)*(kl + (m >> 1));
-            int f = (m & 1) ? v.consR[c] : v.consL[c];
-            cnt[n] = f - v.tr_off[tr] - t;
-         }else if( x == 2 ){          /* same column: the z-track of that column */
-            int tz = P.trz0 + (jl + (m & 1)) + P.Nr*kl;
-            int f = (m >> 1) ? v.consZR[c] : v.consZL[c];
-            cnt[n] = f - v.tr_off[tz] - t;
-         }else{                       /* diagonal: cells of list n before this one */
-            int o = v.ann_off[an[n]], nn = v.ann_np[an[n]], I0n = v.I0[an[n]];
-            /* both lists unrolled from I0: the count is near t nn / np */
-            cnt[n] = gallop_lb(0, nn, __float2int_rz(__fdividef((float)t*(float)nn, (float)np)), [&](int mid){
-               int s = I0n + mid; if( s >= nn ) s -= nn;
-               double uy = v.piph[o + s];
-               return !(n < m ? uy <= ux : uy < ux);
-            });
-         }
+   if( threadIdx.x < 9 ){
+      const int dk = (int)threadIdx.x/3, dj = (int)threadIdx.x%3, jj = j + dj - 1, kk = k + dk - 1;
+      if( jj >= 0 && jj < P.Nr && kk >= 0 && kk < P.Nz ){
+         const int a = P.ann0 + jj + P.Nr*kk;
+         A[dk][dj] = {v.ann_off[a], v.ann_np[a], v.I0[a]};
       }
-      int e = cnt[0] + cnt[1] + cnt[2] + cnt[3];
-      int line = P.ln0 + jl + (P.Nr-1)*kl;
-      if( e < 0 || e >= v.line_off[line+1] - v.line_off[line] ){ err |= ERRF_INTERNAL; continue; }
-      v.rk[m*N + c] = e;
-      /* the reference's state at step e */
-      int cur[4];
-      bool bad = false;
-      for( int n=0 ; n<4 ; ++n ){
-         int o = v.ann_off[an[n]], nn = v.ann_np[an[n]];
-         int s = v.I0[an[n]] + cnt[n];          /* I0 < nn, 0 <= cnt <= nn */
-         if( s >= nn ) s -= nn;
-         if( s < 0 || s >= nn ){ bad = true; s = 0; }
-         cur[n] = o + s;
-      }
-      if( bad ){ err |= ERRF_INTERNAL; continue; }
-      int LR_alt = 0, UD_alt = 0;
-      int w4 = ct_which4(v.piph[cur[0]], v.piph[cur[1]], v.piph[cur[2]], v.piph[cur[3]],
-                         &LR_alt, &UD_alt, 0, Pmax, &err);
-      int w4b = ct_which4(v.piph[cur[0]] - v.dphi[cur[0]], v.piph[cur[1]] - v.dphi[cur[1]],
-                          v.piph[cur[2]] - v.dphi[cur[2]], v.piph[cur[3]] - v.dphi[cur[3]],
-                          NULL, NULL, 1, Pmax, &err);
-      if( w4 != m ) err |= ERRF_INTERNAL;
-      /* E_phi of the cells' owned faces: c [3],[1]; cR [3],[0]; cU [1],[2]; cUR [0],[2] */
-      auto eph = [&](int n, int s){ return ct_ephi(v, P, cur[n], jl + (n & 1), kl + (n >> 1), s); };
-      const R q4 = R(.25);
-      R E;
-      if( w4 == 0 ){
-         E = q4*( eph(0,3) + eph(0,1) );
-         if( LR_alt == 0 ) E += q4*eph(2,1); else E += q4*eph(3,0);
-         if( UD_alt == 0 ) E += q4*eph(1,3); else E += q4*eph(3,2);
-      }else if( w4 == 1 ){
-         E = q4*( eph(1,3) + eph(1,0) );
-         if( LR_alt == 0 ) E += q4*eph(2,1); else E += q4*eph(3,0);
-         if( UD_alt == 0 ) E += q4*eph(0,3); else E += q4*eph(2,2);
-      }else if( w4 == 2 ){
-         E = q4*( eph(2,2) + eph(2,1) );
-         if( LR_alt == 0 ) E += q4*eph(0,1); else E += q4*eph(1,0);
-         if( UD_alt == 0 ) E += q4*eph(1,3); else E += q4*eph(3,2);
-      }else{
-         E = q4*( eph(3,2) + eph(3,0) );
-         if( LR_alt == 0 ) E += q4*eph(0,1); else E += q4*eph(1,0);
-         if( UD_alt == 0 ) E += q4*eph(0,3); else E += q4*eph(2,2);
-      }
-      double xp1 = v.piph[cur[w4]];
-      double xm1 = v.piph[cur[w4b]] - v.dphi[cur[w4b]];
-      double dl = (.5*(rj[jl]+rj[jl]))*get_dp(xp1, xm1, Pmax, &err);   /* get_dL(.,.,0) */
-      v.lineX[v.line_off[line] + e] = (double)E*dl*dt;
+   }else if( threadIdx.x >= 32 && threadIdx.x < 36 ){  /* first faces of the annulus's four tracks */
+      const int s = threadIdx.x - 32;
+      int tr = -1;
+      if( s == 0 && j >= 1 )      tr = P.trr0 + (j-1) + (P.Nr-1)*k;
+      if( s == 1 && j <= P.Nr-2 ) tr = P.trr0 + j + (P.Nr-1)*k;
+      if( s == 2 && k >= 1 )      tr = P.trz0 + j + P.Nr*(k-1);
+      if( s == 3 && k <= P.Nz-2 ) tr = P.trz0 + j + P.Nr*k;
+      s_o[s] = tr >= 0 ? v.tr_off[tr] : 0;
    }
+   __syncthreads();
+   if( i >= np ) return;
+   const int c = b.c0 + i;
+   const double dt = v.ds[b.disk].dt*v.dtfac;
+   int err = 0;
+   int t = i - A[1][1].I0;
+   if( t < 0 ) t += np;
+   const double ux = v.piph[c];
+   const int f4[4] = {v.consR[c], v.consL[c], v.consZR[c], v.consZL[c]};
+   const int o4[4] = {s_o[0], s_o[1], s_o[2], s_o[3]};
+   ct_line_step<0,R>(v, P, A, f4, o4, c, j, k, t, np, ux, dt, &err);
+   ct_line_step<1,R>(v, P, A, f4, o4, c, j, k, t, np, ux, dt, &err);
+   ct_line_step<2,R>(v, P, A, f4, o4, c, j, k, t, np, ux, dt, &err);
+   ct_line_step<3,R>(v, P, A, f4, o4, c, j, k, t, np, ux, dt, &err);
    raise_err(v, err);
 }
 
-/* The edge steps of line l that fall on face f of a track whose two cells'
- * lists in that line are mA (first / inner-lower annulus) and mB: the steps
- * whose pointer sum over the pair equals the face's index d, i.e. after the
- * element that ends face d-1 up to the one that ends face d; face 0 also
- * takes the steps after the pair's last element (the pair has wrapped).
- * Applied in step order as S += sign X. */
+/* The edge steps of line l that fall on face f of a track: the steps whose
+ * pointer sum over the face's pair of lists equals the face's index d, i.e.
+ * after the element that ends face d-1 up to the one that ends face d; face
+ * 0 also takes the steps after the pair's last element (the pair has
+ * wrapped).  slot: which of the face's two lines l is (frk).  Applied in
+ * step order as S += sign X. */
 template<class R>
 __device__ __forceinline__ double ct_line_terms(const ViewT<R> &v, double S, int line, int tr,
-                                                int f, int mA, int mB, double sign){
-   const size_t N = v.Ncell;
+                                                int f, int slot, double sign){
    const double *X = v.lineX + v.line_off[line];
+   const int *rank = v.frk + (size_t)slot*v.Nf;
    int f0 = v.tr_off[tr], f1 = v.tr_off[tr+1];
-   auto rank = [&](int g){
-      return v.fLR[g] == 0 ? v.rk[mA*N + v.fL[g]] : v.rk[mB*N + v.fR[g]];
-   };
-   int hi = rank(f);
-   int lo = f == f0 ? 0 : rank(f-1) + 1;
+   int hi = rank[f];
+   int lo = f == f0 ? 0 : rank[f-1] + 1;
    for( int e=lo ; e<=hi ; ++e ) S += sign*X[e];
    if( f == f0 ){
       int ne = v.line_off[line+1] - v.line_off[line];
-      for( int e=rank(f1-1)+1 ; e<ne ; ++e ) S += sign*X[e];
+      for( int e=rank[f1-1]+1 ; e<ne ; ++e ) S += sign*X[e];
    }
    return S;
 }
@@ -475,27 +500,31 @@ __global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
       const int ln = P.ln0;
       const int W = P.Nr-1;
       if( f2 >= 0 ){                       /* r face (j, j+1) at layer k */
-         if( k >= 1 )      S2 = ct_line_terms(v, S2, ln + j + W*(k-1), t2, f2, 2, 3, -1.0);
-         if( k <= P.Nz-2 ) S2 = ct_line_terms(v, S2, ln + j + W*k, t2, f2, 0, 1, 1.0);
+         if( k >= 1 )      S2 = ct_line_terms(v, S2, ln + j + W*(k-1), t2, f2, 0, -1.0);
+         if( k <= P.Nz-2 ) S2 = ct_line_terms(v, S2, ln + j + W*k, t2, f2, 1, 1.0);
       }
       if( f1 >= 0 ){                       /* r face (j-1, j) at layer k */
-         if( k >= 1 )      S1 = ct_line_terms(v, S1, ln + (j-1) + W*(k-1), t1, f1, 2, 3, -1.0);
-         if( k <= P.Nz-2 ) S1 = ct_line_terms(v, S1, ln + (j-1) + W*k, t1, f1, 0, 1, 1.0);
+         if( k >= 1 )      S1 = ct_line_terms(v, S1, ln + (j-1) + W*(k-1), t1, f1, 0, -1.0);
+         if( k <= P.Nz-2 ) S1 = ct_line_terms(v, S1, ln + (j-1) + W*k, t1, f1, 1, 1.0);
       }
       if( f4 >= 0 ){                       /* z face (k, k+1) of column j */
-         if( j >= 1 )      S4 = ct_line_terms(v, S4, ln + (j-1) + W*k, t4, f4, 1, 3, 1.0);
-         if( j <= P.Nr-2 ) S4 = ct_line_terms(v, S4, ln + j + W*k, t4, f4, 0, 2, -1.0);
+         if( j >= 1 )      S4 = ct_line_terms(v, S4, ln + (j-1) + W*k, t4, f4, 0, 1.0);
+         if( j <= P.Nr-2 ) S4 = ct_line_terms(v, S4, ln + j + W*k, t4, f4, 1, -1.0);
       }
       if( f3 >= 0 ){                       /* z face (k-1, k) of column j */
-         if( j >= 1 )      S3 = ct_line_terms(v, S3, ln + (j-1) + W*(k-1), t3, f3, 1, 3, 1.0);
-         if( j <= P.Nr-2 ) S3 = ct_line_terms(v, S3, ln + j + W*(k-1), t3, f3, 0, 2, -1.0);
+         if( j >= 1 )      S3 = ct_line_terms(v, S3, ln + (j-1) + W*(k-1), t3, f3, 0, 1.0);
+         if( j <= P.Nr-2 ) S3 = ct_line_terms(v, S3, ln + j + W*(k-1), t3, f3, 1, -1.0);
       }
       v.Phi[3*N + c] = S3;
       v.Phi[4*N + c] = S4;
+      if( !first && f3 >= 0 ) v.fPhi[f3] = S3;
+      if( !first && f4 >= 0 ) v.fPhi[f4] = S4;
    }
    v.Phi[N + c] = S1;
    v.Phi[2*N + c] = S2;
    v.Phi[c] = P0;
+   if( !first && f1 >= 0 ) v.fPhi[f1] = S1;
+   if( !first && f2 >= 0 ) v.fPhi[f2] = S2;
    if( first ){
       int err = 0;
       int cprev = c0 + (i == 0 ? np-1 : i-1);
@@ -563,9 +592,9 @@ __global__ void k_ct_flip(ViewT<R> v){
 
 /* B_faces_to_cells type 1 for a real cell (bfields.c:88-309): cons[BRR]
  * (cons[BZZ]) from the fluxes of the cell's r (z) faces -- inner / lower
- * track first, each in face order, slots by the current LRtype -- over their
+ * track first, each in face order -- over their
  * area, cons[BPP] from the two phi faces, with the moved cell's volume */
-template<class R>
+template<class R, bool FACE>
 __device__ void ct_cons_B(const ViewT<R> &v, const DiskParams &P, int a, int c0, int np, int i,
                           int j, int k, double rp, double rm, double zp, double zm, double *cons,
                           int *err){
@@ -573,19 +602,34 @@ __device__ void ct_cons_B(const ViewT<R> &v, const DiskParams &P, int a, int c0,
    int c = c0 + i, cm = c0 + (i == 0 ? np-1 : i-1);
    int I0 = v.I0[a];
    double S = 0.0, T = 0.0;
-   /* every face of the cell's run in its inner (lower) track has the cell as
-    * R, in its outer (upper) track as L; the other side's cell is read only
-    * when that one owns the face */
-   auto sum_rin = [&](int f){
-      S += v.fLR[f] == 0 ? v.Phi[2*N + v.fL[f]] : v.Phi[N + c];
-      T += v.fdA[f];
-   };
-   auto sum_rout = [&](int f){
-      S += v.fLR[f] == 0 ? v.Phi[2*N + c] : v.Phi[N + v.fR[f]];
-      T += v.fdA[f];
-   };
-   if( j >= 1 )      ct_over_runs(v, v.consR, P.trr0 + (j-1) + (P.Nr-1)*k, c0, np, i, I0, sum_rin);
-   if( j <= P.Nr-2 ) ct_over_runs(v, v.consL, P.trr0 + j + (P.Nr-1)*k, c0, np, i, I0, sum_rout);
+   double Sz = 0.0, Tz = 0.0;
+   const bool z3 = v.ct == 2 && P.Nz > 1;
+   const int tri = P.trr0 + (j-1) + (P.Nr-1)*k, tro = P.trr0 + j + (P.Nr-1)*k;
+   const int tzi = P.trz0 + j + P.Nr*(k-1), tzo = P.trz0 + j + P.Nr*k;
+   if( FACE && v.topo_set ){
+      /* no flips since k_ct_update (the second substep): the fluxes face by
+       * face (fPhi), a run being two streams of consecutive loads */
+      auto sum = [&](int f){ S += v.fPhi[f]; T += v.fdA[f]; };
+      auto zsum = [&](int f){ Sz += v.fPhi[f]; Tz += v.fdA[f]; };
+      if( j >= 1 )      ct_over_runs(v, v.consR, tri, c0, np, i, I0, sum);
+      if( j <= P.Nr-2 ) ct_over_runs(v, v.consL, tro, c0, np, i, I0, sum);
+      if( z3 && k >= 1 )      ct_over_runs(v, v.consZR, tzi, c0, np, i, I0, zsum);
+      if( z3 && k <= P.Nz-2 ) ct_over_runs(v, v.consZL, tzo, c0, np, i, I0, zsum);
+   }else{
+      /* through the slot of each face's owner by its LRtype, which flips may
+       * have toggled (several faces can name one slot then): every face of
+       * the cell's run in its inner (lower) track has the cell as R, in its
+       * outer (upper) track as L; the other side's cell is read only when
+       * that one owns the face */
+      auto sum_in = [&](int f){ S += v.fLR[f] == 0 ? v.Phi[2*N + v.fL[f]] : v.Phi[N + c]; T += v.fdA[f]; };
+      auto sum_out = [&](int f){ S += v.fLR[f] == 0 ? v.Phi[2*N + c] : v.Phi[N + v.fR[f]]; T += v.fdA[f]; };
+      auto sum_zin = [&](int f){ Sz += v.fLR[f] == 0 ? v.Phi[4*N + v.fL[f]] : v.Phi[3*N + c]; Tz += v.fdA[f]; };
+      auto sum_zout = [&](int f){ Sz += v.fLR[f] == 0 ? v.Phi[4*N + c] : v.Phi[3*N + v.fR[f]]; Tz += v.fdA[f]; };
+      if( j >= 1 )      ct_over_runs(v, v.consR, tri, c0, np, i, I0, sum_in);
+      if( j <= P.Nr-2 ) ct_over_runs(v, v.consL, tro, c0, np, i, I0, sum_out);
+      if( z3 && k >= 1 )      ct_over_runs(v, v.consZR, tzi, c0, np, i, I0, sum_zin);
+      if( z3 && k <= P.Nz-2 ) ct_over_runs(v, v.consZL, tzo, c0, np, i, I0, sum_zout);
+   }
    double x0 = v.ann_rc[a];                          /* centroid_r(rp, rm) */
    double dph = get_dp(v.piph[c], v.piph[cm], P.Pmax, err);
    double dV = dV_of(rp, rm, dph, zp, zm);
@@ -594,18 +638,7 @@ __device__ void ct_cons_B(const ViewT<R> &v, const DiskParams &P, int a, int c0,
    double hr = 1.0, hp = x0;
    cons[BRR] = S * (dV*rfac/(T * hr));
    cons[BPP] = .5*(v.Phi[c]+v.Phi[cm])*dV/(dA * hp);
-   if( v.ct == 2 && P.Nz > 1 ){
-      double Sz = 0.0, Tz = 0.0;
-      auto sum_zin = [&](int f){
-         Sz += v.fLR[f] == 0 ? v.Phi[4*N + v.fL[f]] : v.Phi[3*N + c];
-         Tz += v.fdA[f];
-      };
-      auto sum_zout = [&](int f){
-         Sz += v.fLR[f] == 0 ? v.Phi[4*N + c] : v.Phi[3*N + v.fR[f]];
-         Tz += v.fdA[f];
-      };
-      if( k >= 1 )      ct_over_runs(v, v.consZR, P.trz0 + j + P.Nr*(k-1), c0, np, i, I0, sum_zin);
-      if( k <= P.Nz-2 ) ct_over_runs(v, v.consZL, P.trz0 + j + P.Nr*k, c0, np, i, I0, sum_zout);
+   if( z3 ){
       double zfac = 1.0, hz = 1.0;                      /* bfield_scale_factor(x2, 2) */
       cons[BZZ] = Sz * (dV*zfac/(Tz * hz));
    }

@@ -181,11 +181,12 @@ struct ViewT {
     * averaging (FP32 in the mixed form, whose face fluxes stay FP64); pE, pB, pEr, pBz the phi face's (Ez, Br, Er, Bz) from
     * flux_to_E.  Per face (r and z): fEt / fBt (Erz, Brz), fEphi (E_phi),
     * fX the E dl dt of update_B_fluxes, fFlip the flag of check_flipped.
-    * 3D: rk[m*Ncell + c] the position of cell c in the 4-way merge of the
-    * edge line where it is list m (make_edge_adjust's c, cR, cU, cUR), and
-    * lineX[line_off[l] + e] the E_phi dl dt of merged edge e of line l. */
+    * 3D: frk[s*Nf + f] the position, in the 4-way merge of an edge line that
+    * face f borders (s = 0 the lower / inner one, 1 the upper / outer one), of
+    * the cell that ends the face, and lineX[line_off[l] + e] the E_phi dl dt of merged edge e of line l. */
    int ct, nfs;
    double *Phi, *RKPhi, *fX;            /* the face fluxes stay FP64 in both forms */
+   double *fPhi;                        /* each face's flux after the second substep's update */
    /* grmhd2: the metric at the fixed points where the step evaluates it
     * (k_gr_tables; NULL for the Newtonian modules) */
    GRAnn *gr_ann;
@@ -202,7 +203,7 @@ struct ViewT {
     * E (avg_Efields' z-pole average, k_ct_zpole); NULL otherwise */
    double *ctPole;
    unsigned char *fFlip;
-   int *rk, *line_off;
+   int *frk, *line_off;
    double *lineX;
 };
 
@@ -1521,7 +1522,7 @@ __device__ __forceinline__ bool fixed_ghost_init(const DiskParams &P, int bc, in
 }
 
 /* B_faces_to_cells type 1 under constrained transport (disco_ct.cuh) */
-template<class R>
+template<class R, bool FACE>
 __device__ void ct_cons_B(const ViewT<R> &v, const DiskParams &P, int a, int c0, int np, int i,
                           int j, int k, double rp, double rm, double zp, double zm, double *cons,
                           int *err);
@@ -1674,7 +1675,7 @@ __device__ __forceinline__ void c2p_tail(const ViewT<R> &v, const DiskParams &P,
 /* ------------------------------------------------------------------ k_c2p
  * c2p_tail on each cell after k_update, with constrained transport first
  * rebuilding B from the face fluxes (onestep.c:183-185). */
-template<int Q, int NC, class R, int NQD = 5, bool VISC = false, bool GR = false>
+template<int Q, int NC, class R, int NQD = 5, bool VISC = false, bool GR = false, bool FACE = true>
 __device__ __forceinline__ void c2p_body(const ViewT<R> &v, int last, int bc, int diag, int move_c2p,
                                          int topo_set, int bid){
    const CellBlk b = v.cblk[bid];
@@ -1705,7 +1706,7 @@ __device__ __forceinline__ void c2p_body(const ViewT<R> &v, int last, int bc, in
             if( v.ct ){                  /* onestep.c:183-185 */
                const double *rj = v.rj + P.rj0 + 1;
                const double *zk = v.zk + P.zk0 + 1;
-               ct_cons_B(v, P, a, c0, np, i, j, k, rj[j], rj[j-1], zk[k], zk[k-1], cons, &err);
+               ct_cons_B<R,FACE>(v, P, a, c0, np, i, j, k, rj[j], rj[j-1], zk[k], zk[k-1], cons, &err);
                v.cons[BRR*N + c] = cons[BRR];
                v.cons[BPP*N + c] = cons[BPP];
                if( v.ct == 2 && P.Nz > 1 ) v.cons[BZZ*N + c] = cons[BZZ];
@@ -1721,7 +1722,7 @@ __device__ __forceinline__ void c2p_body(const ViewT<R> &v, int last, int bc, in
  * substeps without the reductions keep fewer registers */
 template<int Q, int NC, class R, int NQD = 5, bool VISC = false, bool GR = false, int LAST = 1>
 __global__ void __launch_bounds__(CB, GR ? MB_GR_LIGHT : (Q > 6 ? MB_MHD_C2P : MB_C2P)) k_c2p(ViewT<R> v, int bc, int diag){
-   c2p_body<Q,NC,R,NQD,VISC,GR>(v, LAST, bc, diag, v.move_c2p, v.topo_set, blockIdx.x);
+   c2p_body<Q,NC,R,NQD,VISC,GR,LAST != 0>(v, LAST, bc, diag, v.move_c2p, v.topo_set, blockIdx.x);
 }
 
 /* The sequential walk of set_cells_copy_distant (boundary_functions.c:
