@@ -185,18 +185,32 @@ static void launch_c2p(disco_batch *b, const ViewT<R> &v, int last, int diag){
    if( b->nq == 8 ) launch_c2p_nq<Q,NC,R,8,GR>(b, v, last, diag);
    else launch_c2p_nq<Q,NC,R,5,GR>(b, v, last, diag);
 }
-/* trans_flux of one direction, only the blocks of its tracks with fluxes
- * (one launch for both compiled the two solves into one register budget:
- * the GRMHD step slowed by 6%) */
-template<int Q, int NC, int DIM, class R, bool GR = false>
+/* trans_flux, only the blocks of tracks with fluxes, of both directions in
+ * one launch (a 41 x 25-annulus MHD step of 400 us lost 4% to the second) --
+ * except grmhd2's, whose solve fills the register budget: compiled twice into
+ * one kernel it spilled more and cost the GRMHD step 6% */
+template<int Q, int NC, class R, bool GR = false>
 static void launch_flux_t(disco_batch *b, const ViewT<R> &v0){
-   const unsigned nfb = DIM == 1 ? (unsigned)b->nfl_r : (unsigned)b->fblk_fl.size() - b->nfl_r;
+   unsigned nfb = (unsigned)b->fblk_fl.size();
    if( nfb == 0 ) return;
-   ViewT<R> v = v0; v.fblk = b->d_fblk_fl + (DIM == 1 ? 0 : b->nfl_r);
+   cudaStream_t s = b->stream;
+   ViewT<R> v = v0; v.fblk = b->d_fblk_fl;
    if constexpr ( NC == 5 ){
-      if( b->any_visc ){ k_flux_t<Q,NC,DIM,R,true><<<nfb, FB, 0, b->stream>>>(v); return; }
+      if( b->any_visc ){
+         if( b->any_3d ) k_flux_t<Q,NC,3,R,true><<<nfb, FB, 0, s>>>(v, b->nfl_r);
+         else            k_flux_t<Q,NC,1,R,true><<<nfb, FB, 0, s>>>(v, b->nfl_r);
+         return;
+      }
    }
-   k_flux_t<Q,NC,DIM,R,false,GR><<<nfb, FB, 0, b->stream>>>(v);
+   if constexpr ( GR ){
+      const unsigned nr = (unsigned)b->nfl_r;
+      if( nr > 0 ) k_flux_t<Q,NC,1,R,false,GR><<<nr, FB, 0, s>>>(v, 0);
+      v.fblk += nr;
+      if( nfb > nr ) k_flux_t<Q,NC,2,R,false,GR><<<nfb - nr, FB, 0, s>>>(v, 0);
+   }else{
+      if( b->any_3d ) k_flux_t<Q,NC,3,R,false,GR><<<nfb, FB, 0, s>>>(v, b->nfl_r);
+      else            k_flux_t<Q,NC,1,R,false,GR><<<nfb, FB, 0, s>>>(v, b->nfl_r);
+   }
 }
 
 /* One substep of onestep() (onestep.c:84-229); GR: the grmhd2 module. */
@@ -224,8 +238,7 @@ static void launch_substep(disco_batch *b, ViewT<R> v, int first, int last, doub
    const unsigned nwm = first && b->any_mm3 ? nblk(v.Nann, WM_WARPS) : 0;
    if( b->any_3d ){ k_grad<Q,true,R><<<nwm + ncb, CB, 0, s>>>(v, (int)nwm);  mark(b, "k_grad"); }
    else{            k_grad<Q,false,R><<<nwm + ncb, CB, 0, s>>>(v, (int)nwm); mark(b, "k_gradr"); }
-   launch_flux_t<Q,NC,1,R,GR>(b, v);                   mark(b, "k_flux_r");
-   if( b->any_3d ){ launch_flux_t<Q,NC,2,R,GR>(b, v);  mark(b, "k_flux_z"); }
+   launch_flux_t<Q,NC,R,GR>(b, v);                     mark(b, b->any_3d ? "k_flux" : "k_flux_r");
    bool upd_visc = false;
    if constexpr ( NC == 5 ) upd_visc = b->any_visc;
    if( upd_visc ){

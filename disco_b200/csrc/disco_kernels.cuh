@@ -900,9 +900,12 @@ __device__ __forceinline__ void flux_body(const ViewT<R> &v, double dtfac, int b
    for( int q=0 ; q<Q ; ++q ) v.fG[(size_t)q*v.Nf + f] = G[q];
    raise_err(v, err);
 }
-template<int Q, int NC, int DIM, class R, bool VISC = false, bool GR = false>
-__global__ void __launch_bounds__(FB, GR ? MB_GR : (Q > 6 ? MB_MHD_FLUX : MB_FLUX)) k_flux_t(ViewT<R> v){
-   flux_body<Q,NC,DIM,R,VISC,GR>(v, v.dtfac, blockIdx.x);
+/* the blocks of v.fblk: DIRS 1 of r tracks, 2 of z tracks, 3 the first nr
+ * of r tracks and the rest of z tracks */
+template<int Q, int NC, int DIRS, class R, bool VISC = false, bool GR = false>
+__global__ void __launch_bounds__(FB, GR ? MB_GR : (Q > 6 ? MB_MHD_FLUX : MB_FLUX)) k_flux_t(ViewT<R> v, int nr){
+   if( DIRS == 1 || (DIRS == 3 && (int)blockIdx.x < nr) ) flux_body<Q,NC,1,R,VISC,GR>(v, v.dtfac, blockIdx.x);
+   else if constexpr ( DIRS != 1 ) flux_body<Q,NC,2,R,VISC,GR>(v, v.dtfac, blockIdx.x);
 }
 
 /* ------------------------------------------------------------------ phi faces
