@@ -89,27 +89,40 @@ __device__ __forceinline__ void gr_flux(const GRParams &G, const Metric3 &g, con
    F[8] = prim[8]*F[DDD];
 }
 
+/* gamma^ij l_j and w = sqrt(1 + l_i l^i) of one state: vel(), flux() and
+ * prim2cons() each evaluate them with these expressions */
+struct GRSide { double igaml[3], u2, w; };
+__device__ __forceinline__ GRSide gr_side(const Metric3 &g, const double *prim){
+   GRSide s;
+   const double l[3] = {prim[URR], prim[UPP], prim[UZZ]};
+   s.u2 = 0.0;
+#pragma unroll
+   for( int i=0 ; i<3 ; ++i ){
+      s.igaml[i] = 0.0;
+#pragma unroll
+      for( int j=0 ; j<3 ; ++j ) s.igaml[i] += g.igam[3*i+j]*l[j];
+      s.u2 += s.igaml[i]*l[i];
+   }
+   s.w = sqrt(1.0 + s.u2);
+   return s;
+}
+
 /* flux() and prim2cons(dV = 1) of the same state at the same point: the two
  * reference functions compute the same intermediates (u^i, w, b^mu, b^2,
  * ...) with the same expressions, so evaluating them once gives both results
  * bit for bit */
-__device__ __forceinline__ void gr_flux_cons(const GRParams &G, const Metric3 &g, const double *prim,
-                                             const double *x, const double *n, double *F, double *Uc){
+__device__ __forceinline__ void gr_flux_cons(const GRParams &G, const Metric3 &g, const GRSide &sd,
+                                             const double *prim, const double *x, const double *n,
+                                             double *F, double *Uc){
    const double r = x[0];
    const double al = g.al, jac = g.jac, sqrtgam = g.sqrtgam;
-   const double *be = g.be, *gam = g.gam, *igam = g.igam, *U = g.U;
+   const double *be = g.be, *gam = g.gam, *U = g.U;
    const double rho = prim[RHO], Pp = prim[PPP];
    const double l[3] = {prim[URR], prim[UPP], prim[UZZ]};
    const double B[3] = {prim[BRR]/sqrtgam, prim[BPP]/(r*sqrtgam), prim[BZZ]/sqrtgam};
-   double igaml[3], u[3], v[3];
-#pragma unroll
-   for( int i=0 ; i<3 ; ++i ){
-      igaml[i] = 0.0;
-#pragma unroll
-      for( int j=0 ; j<3 ; ++j ) igaml[i] += igam[3*i+j]*l[j];
-   }
-   const double u2 = l[0]*igaml[0] + l[1]*igaml[1] + l[2]*igaml[2];
-   const double w = sqrt(1.0 + u2);
+   const double *igaml = sd.igaml;
+   double u[3], v[3];
+   const double w = sd.w;
    const double u0 = w/al;
 #pragma unroll
    for( int i=0 ; i<3 ; ++i ) u[i] = igaml[i] - be[i]*u0;
@@ -167,23 +180,18 @@ __device__ __forceinline__ void gr_flux_cons(const GRParams &G, const Metric3 &g
 
 /* ------------------------------------------------------------- HLL speeds */
 /* one side's fast speeds along n (grmhd2.c:551-612 for one of the two states) */
-__device__ __forceinline__ void gr_side_speeds(const GRParams &G, const Metric3 &g, double sqrtgam_v,
-                                               const double *prim, const double *n, double r,
+__device__ __forceinline__ void gr_side_speeds(const GRParams &G, const Metric3 &g, const GRSide &sd,
+                                               double sqrtgam_v, const double *prim, const double *n, double r,
                                                double bn, double ign, double hn,
                                                double *sl, double *sr){
    const double gl = G.gam;
-   const double *gam = g.gam, *igam = g.igam;
+   const double *gam = g.gam;
    const double rho = prim[RHO], P = prim[PPP];
    const double l[3] = {prim[URR], prim[UPP], prim[UZZ]};
    const double B[3] = {prim[BRR]/sqrtgam_v, prim[BPP]/(r*sqrtgam_v), prim[BZZ]/sqrtgam_v};
    const double cs2 = gl*P/(rho+gl/(gl-1.0)*P);
-   double uS[3], u2 = 0.0;
-   for( int i=0 ; i<3 ; ++i ){
-      uS[i] = 0.0;
-      for( int j=0 ; j<3 ; ++j ) uS[i] += igam[3*i+j]*l[j];
-      u2 += uS[i]*l[i];
-   }
-   const double w = sqrt(1.0+u2);
+   const double *uS = sd.igaml;
+   const double u2 = sd.u2, w = sd.w;
    const double v2 = u2/(w*w);
    const double uB = l[0]*B[0] + l[1]*B[1] + l[2]*B[2];
    double B2 = 0.0;
@@ -199,7 +207,8 @@ __device__ __forceinline__ void gr_side_speeds(const GRParams &G, const Metric3 
 }
 
 /* vel()'s Sl, Sr (the contact speed it also returns only serves HLLC) */
-__device__ __forceinline__ void gr_hll_speeds(const GRParams &G, const Metric3 &g, const double *primL,
+__device__ __forceinline__ void gr_hll_speeds(const GRParams &G, const Metric3 &g, const GRSide &sL,
+                                              const GRSide &sR, const double *primL,
                                               const double *primR, const double *n, const double *x,
                                               double *Sl, double *Sr){
    const double r = x[0];
@@ -208,8 +217,8 @@ __device__ __forceinline__ void gr_hll_speeds(const GRParams &G, const Metric3 &
    const double ign = g.igam[3*0+0]*n[0] + g.igam[3*1+1]*n[1] + g.igam[3*2+2]*n[2];
    const double hn = n[0] + r*n[1] + n[2];
    double sl1, sr1, sl2, sr2;
-   gr_side_speeds(G, g, sqrtgam_v, primL, n, r, bn, ign, hn, &sl1, &sr1);
-   gr_side_speeds(G, g, sqrtgam_v, primR, n, r, bn, ign, hn, &sl2, &sr2);
+   gr_side_speeds(G, g, sL, sqrtgam_v, primL, n, r, bn, ign, hn, &sl1, &sr1);
+   gr_side_speeds(G, g, sR, sqrtgam_v, primR, n, r, bn, ign, hn, &sl2, &sr2);
    *Sr = sr1 > sr2 ? sr1 : sr2;
    *Sl = sl1 < sl2 ? sl1 : sl2;
 }
@@ -222,18 +231,19 @@ __device__ __forceinline__ void gr_hll(const DiskParams &P, const Metric3 &g, co
                                        const double *primR, const double *x, const double *n,
                                        double w, double dAdt, double *Gq){
    const GRParams G = gr_params(P);
+   const GRSide sL = gr_side(g, primL), sR = gr_side(g, primR);
    double Sl, Sr;
-   gr_hll_speeds(G, g, primL, primR, n, x, &Sl, &Sr);
+   gr_hll_speeds(G, g, sL, sR, primL, primR, n, x, &Sl, &Sr);
    double Flux[GR_Q], Ustr[GR_Q];
    if( w < Sl ){
-      gr_flux_cons(G, g, primL, x, n, Flux, Ustr);
+      gr_flux_cons(G, g, sL, primL, x, n, Flux, Ustr);
    }else if( w > Sr ){
-      gr_flux_cons(G, g, primR, x, n, Flux, Ustr);
+      gr_flux_cons(G, g, sR, primR, x, n, Flux, Ustr);
    }else{
       double Fl[GR_Q], Fr[GR_Q], Ul[GR_Q], Ur[GR_Q];
       const double aL = Sr, aR = -Sl;
-      gr_flux_cons(G, g, primL, x, n, Fl, Ul);
-      gr_flux_cons(G, g, primR, x, n, Fr, Ur);
+      gr_flux_cons(G, g, sL, primL, x, n, Fl, Ul);
+      gr_flux_cons(G, g, sR, primR, x, n, Fr, Ur);
 #pragma unroll
       for( int q=0 ; q<GR_Q ; ++q ){
          Flux[q] = ( aL*Fl[q] + aR*Fr[q] + aL*aR*( Ul[q] - Ur[q] ) )/( aL + aR );
