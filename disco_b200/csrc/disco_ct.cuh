@@ -461,9 +461,10 @@ __global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
    auto fm_of = [&](int f, int tr){ return f > v.tr_off[tr] ? f-1 : v.tr_off[tr+1]-1; };
    /* the RK snapshot / average of the slots (timestep.c:22, adjust_RK_cons
     * misc.c:239-241), taken here as their one read before the update */
-   auto start = [&](int s){ return rk_start(v.Phi, v.RKPhi, s*N + c, first); };
-   double P0 = start(0);
-   double S1 = start(1), S2 = start(2), S3 = 0.0, S4 = 0.0;
+   double st[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+   if( z3 ) rk_start<5>(v.Phi, v.RKPhi, N, c, first, st);
+   else     rk_start<3>(v.Phi, v.RKPhi, N, c, first, st);
+   double P0 = st[0], S1 = st[1], S2 = st[2], S3 = st[3], S4 = st[4];
    int f1 = -1, f2 = -1, f3 = -1, f4 = -1, t1 = 0, t2 = 0, t3 = 0, t4 = 0;
    if( j >= 1 ){                           /* inner r face: owned with LRtype 1 */
       t1 = P.trr0 + (j-1) + (P.Nr-1)*k;
@@ -480,7 +481,6 @@ __global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
       S2 = f2 > v.tr_off[t2] ? (S2 + X[fm]) - X[f2] : (S2 - X[f2]) + X[fm];
    }
    if( z3 ){
-      S3 = start(3); S4 = start(4);
       if( k >= 1 ){                        /* lower z face: LRtype 1, R->Phi[3] += X */
          t3 = P.trz0 + j + P.Nr*(k-1);
          f3 = v.consZR[c];

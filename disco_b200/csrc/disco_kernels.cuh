@@ -492,6 +492,34 @@ __device__ __forceinline__ int gallop_lb(int lo, int hi, int g, Pr p){
  * slopes S_q of plm_trans (plm.c:82-89) when with_slopes is set: the
  * gather reads each twice (sum, limiter), and recomputing them there from
  * the two cells' scattered states was measured 5x slower than storing. */
+/* The PLM face slopes S_q of plm_trans (plm.c:82-89).  In the mixed build all
+ * loads come before the first store: the compiler may not move a load over a
+ * store that might alias it, so loaded and stored field by field the fields
+ * are Q round trips to memory in a row (k_faces, 32 disks of binary_nz:
+ * 2.81 -> 2.51 ms per step; 64 disks of 5k..100k cells 0.570 -> 0.530).  FP64
+ * keeps the round trips: Q slopes of 64 bits do not fit in the registers that
+ * 16 blocks per SM leave a thread, and fewer blocks cost more than that
+ * (0.782 field by field, 0.911 together, 1.014 together at 10 blocks). */
+template<int Q, class R>
+__device__ __forceinline__ void face_slopes(const ViewT<R> &v, int cL, int cR, R dpL, R dpR, R dxL, R dxR, int f){
+   const int N = v.Ncell;
+   auto slope = [&](int q){
+      R WL = v.prim[q*N + cL] + dpL*v.gradp[q*N + cL];
+      R WR = v.prim[q*N + cR] - dpR*v.gradp[q*N + cR];
+      return (WR-WL)/(dxR+dxL);
+   };
+   if constexpr ( sizeof(R) == sizeof(float) ){
+      R S[Q];
+#pragma unroll
+      for( int q=0 ; q<Q ; ++q ) S[q] = slope(q);
+#pragma unroll
+      for( int q=0 ; q<Q ; ++q ) v.fS[(size_t)q*v.Nf + f] = S[q];
+   }else{
+#pragma unroll
+      for( int q=0 ; q<Q ; ++q ) v.fS[(size_t)q*v.Nf + f] = slope(q);
+   }
+}
+
 template<int Q, class R>
 __device__ __forceinline__ void faces_body(const ViewT<R> &v, int with_slopes, int topo_reuse, int bid){
    const FaceBlk b = v.fblk[bid];
@@ -515,12 +543,7 @@ __device__ __forceinline__ void faces_body(const ViewT<R> &v, int with_slopes, i
       double phiL = v.piph[cL] - .5*v.dphi[cL], phiR = v.piph[cR] - .5*v.dphi[cR];
       R dpL = (R)get_signed_dp(phic, phiL, Pmax, &err);
       R dpR = (R)get_signed_dp(phiR, phic, Pmax, &err);
-#pragma unroll
-      for( int q=0 ; q<Q ; ++q ){
-         R WL = v.prim[q*N + cL] + dpL*v.gradp[q*N + cL];
-         R WR = v.prim[q*N + cR] - dpR*v.gradp[q*N + cR];
-         v.fS[(size_t)q*v.Nf + f] = (WR-WL)/(dxR+dxL);
-      }
+      face_slopes<Q,R>(v, cL, cR, dpL, dpR, dxL, dxR, f);
       raise_err(v, err);
       return;
    }
@@ -569,23 +592,22 @@ __device__ __forceinline__ void faces_body(const ViewT<R> &v, int with_slopes, i
       dA = r*dr*dp;                                       /* get_dA(.,.,2) */
    }
 
-   v.fL[f] = cL; v.fR[f] = cR; v.fLR[f] = (unsigned char)LR;
-   v.fphic[f] = phic; v.fdA[f] = dA; v.fdp[f] = dp;
-   if( b.dim == 1 ){ if( LR == 0 ) v.consL[cL] = f; else v.consR[cR] = f; }
-   else                  { if( LR == 0 ) v.consZL[cL] = f; else v.consZR[cR] = f; }
-
+   auto store_topo = [&](){
+      v.fL[f] = cL; v.fR[f] = cR; v.fLR[f] = (unsigned char)LR;
+      v.fphic[f] = phic; v.fdA[f] = dA; v.fdp[f] = dp;
+      if( b.dim == 1 ){ if( LR == 0 ) v.consL[cL] = f; else v.consR[cR] = f; }
+      else                  { if( LR == 0 ) v.consZL[cL] = f; else v.consZR[cR] = f; }
+   };
+   if constexpr ( sizeof(R) == sizeof(double) ) store_topo();
    if( with_slopes ){
       R dxL = (R)v.tr_dxL[t], dxR = (R)v.tr_dxR[t];
       double phiL = pL - .5*dL, phiR = pR - .5*dR;
       R dpL = (R)get_signed_dp(phic, phiL, Pmax, &err);
       R dpR = (R)get_signed_dp(phiR, phic, Pmax, &err);
-#pragma unroll
-      for( int q=0 ; q<Q ; ++q ){
-         R WL = v.prim[q*N + cL] + dpL*v.gradp[q*N + cL];
-         R WR = v.prim[q*N + cR] - dpR*v.gradp[q*N + cR];
-         v.fS[(size_t)q*v.Nf + f] = (WR-WL)/(dxR+dxL);
-      }
+      face_slopes<Q,R>(v, cL, cR, dpL, dpR, dxL, dxR, f);
    }
+   if constexpr ( sizeof(R) == sizeof(float) ) store_topo();
+
    raise_err(v, err);
 }
 template<int Q, class R>
@@ -977,16 +999,26 @@ __device__ __forceinline__ QVec<Q,R> phi_face_flux_visc(const ViewT<R> &v, const
 }
 
 /* The RK snapshot of the first substep (timestep.c:18-24: RK_x = x) or the
- * average of the second (adjust_RK_cons, misc.c:226-244, RK = 1/2), element
- * o of x; returns the value the substep's update starts from.  In the first
- * (RK = 0) that is x itself, bit for bit, unless x is not finite. */
-__device__ __forceinline__ double rk_start(const double *x, double *RKx, size_t o, int first){
-   const double xo = x[o];
+ * average of the second (adjust_RK_cons, misc.c:226-244, RK = 1/2) of M rows
+ * of x at c: the values the substep's update starts from, into x0.  In the
+ * first (RK = 0) these are x itself, bit for bit, unless not finite.  Every
+ * row is loaded before the first is stored (see face_slopes): k_update, ms per
+ * step, 64 disks 1.031 -> 0.996 (mixed 1.009 -> 0.940), MHD 64x64 annuli
+ * 0.637 -> 0.599; k_ct_update of 32 disks of binary_nz 2.147 -> 1.870. */
+template<int M>
+__device__ __forceinline__ void rk_start(const double *x, double *RKx, size_t N, size_t c, int first, double *x0){
+#pragma unroll
+   for( int q=0 ; q<M ; ++q ) x0[q] = x[q*N + c];
    if( first ){
-      RKx[o] = xo;
-      return isfinite(xo) ? xo : xo + 0.0*xo;
+#pragma unroll
+      for( int q=0 ; q<M ; ++q ){
+         RKx[q*N + c] = x0[q];
+         if( !isfinite(x0[q]) ) x0[q] = x0[q] + 0.0*x0[q];
+      }
+   }else{
+#pragma unroll
+      for( int q=0 ; q<M ; ++q ) x0[q] = (1.-.5)*x0[q] + .5*RKx[q*N + c];
    }
-   return (1.-.5)*xo + .5*RKx[o];
 }
 
 /* ------------------------------------------------------------------ k_update
@@ -1126,13 +1158,13 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       double cons[Q], cc[Q];
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ){
-         cons[q] = rk_start(v.cons, v.RKcons, (size_t)q*N + c, first);
          if constexpr ( sizeof(R) != sizeof(double) ){
             /* the carry belongs to cons; averaged with it (RKcons keeps none) */
             cc[q] = (double)v.ccarry[q*N + c];
             if( !first ) cc[q] = (double)(float)(.5*cc[q]);
          }else cc[q] = 0.0;
       }
+      rk_start<Q>(v.cons, v.RKcons, N, c, first, cons);
       /* The face fluxes: in the FP64 path added to cons one by one in the
        * reference's order; in the mixed form (FP32 fluxes) summed in a plain
        * FP64 accumulator, exact for a handful of FP32 values whose exponents
@@ -1263,8 +1295,8 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       }
    }
    else if( first ){                /* a ghost's cons is not evolved: its snapshot alone */
-#pragma unroll
-      for( int q=0 ; q<Q ; ++q ) v.RKcons[q*N + c] = v.cons[q*N + c];
+      double x0[Q];
+      rk_start<Q>(v.cons, v.RKcons, N, c, first, x0);
    }
    /* the move follows in k_c2p (or k_ct_update) */
    raise_err(v, err);

@@ -20,6 +20,10 @@
  *          k_update     1.1315   0.9534   0.9760   1.0558   1.6486   -> 8
  *          k_c2p        0.5651   0.4731   0.4832   0.4763   0.5304   -> 8
  *
+ * k_faces of the mixed build since loads all its fields before it stores one
+ * and takes 12 (0.530 at 16, 0.530 at 12 here; 2.652 and 2.509 on 32 disks of
+ * the 3D binary).
+ *
  * Values given with -D on the command line win.
  */
 #pragma once
@@ -34,7 +38,7 @@
 #define MB_BEGIN 16
 #endif
 #ifndef MB_FACES
-#define MB_FACES 16
+#define MB_FACES 12
 #endif
 #ifndef MB_GRAD
 #define MB_GRAD 16
