@@ -71,7 +71,8 @@ def kernel_bytes(name, first, N, Nf, Na, nreal=0):
     if name == "k_step":
         return B_ALG_STEP * nreal
     if name == "k_begin":
-        return N * w * ((5 * Q + 4) if first else (5 * Q + 1))
+        # prim, dphi -> gradp (+ piph -> wiph, piph_new in the first substep)
+        return N * w * ((2 * Q + 4) if first else (2 * Q + 1))
     if name == "k_c2p":
         # reads cons, piph, dphi (+wiph on the last substep); writes prim
         return N * w * (2 * Q + 2) + (N * w if not first else 0)
@@ -92,9 +93,9 @@ def kernel_bytes(name, first, N, Nf, Na, nreal=0):
         return Nf * (4 + 4 + 2 * w + Q * w) + N * w * (3 * Q + 2)
     if name == "k_update":
         # reads cons, prim, gradp (phi faces), piph, dphi, wiph, the consume
-        # indices and the r-face fluxes; writes cons (+ piph_new -> piph,
-        # dphi in the first substep)
-        return N * w * (4 * Q + (6 if first else 3)) + N * 8 + Nf * w * Q
+        # indices and the r-face fluxes; writes cons; RKcons written in the
+        # first substep and read in the second
+        return N * w * (5 * Q + 3) + N * 8 + Nf * w * Q
     return 0
 
 
@@ -110,22 +111,24 @@ def kernel_bytes_mhd(name, first, N, Nfr, Nfz, mixed):
     ck = 4 if mixed else 0               # Kahan carry per conserved variable
     phi = 5 * w
     if name == "k_update":
-        # cons (+carry) read and written, prim and gradp, piph / dphi / wiph,
-        # the four consume indices, the phi-face EMFs written (4); the r- and
+        # cons (+carry) read and written, RKcons written (first) or read,
+        # prim and gradp, piph / dphi / wiph, the four consume indices, the phi-face EMFs written (4); the r- and
         # z-face fluxes read
-        return N * (2 * q * (w + ck) + 2 * q * wr + 3 * w + 16 + 4 * wr) + (Nfr + Nfz) * q * wr
+        return N * (2 * q * (w + ck) + q * w + 2 * q * wr + 3 * w + 16 + 4 * wr) + (Nfr + Nfz) * q * wr
     if name in ("k_flux_r", "k_flux_z"):
         nf = Nfr if name == "k_flux_r" else Nfz
         # per face: its two cells, its geometry, the flux and the two edge
         # terms written; per cell once: prim, the slope in this direction, gradp
         return nf * (8 + 3 * w + q * wr + 2 * wr) + N * (3 * q * wr + 2 * w)
+    if name == "k_flux":
+        # r and z in one launch: prim and gradp once, both slopes
+        return (Nfr + Nfz) * (8 + 3 * w + q * wr + 2 * wr) + N * (4 * q * wr + 2 * w)
     if name == "k_c2p":
         # cons (+carry), piph / dphi (moved in the first substep), the face
         # fluxes rebuilt into the cell field, the prims written (+wiph last)
         return N * (q * (w + ck) + 2 * w + phi + 3 * w + q * wr) + (0 if first else N * w)
     if name == "k_begin":
-        rk = q * w if first else q * (w + 2 * ck)
-        return N * (2 * q * wr + 2 * q * w + rk + 2 * w + (2 * w if first else 0) + 3 * phi)
+        return N * (2 * q * wr + w + (3 * w if first else 0))
     if name in ("k_gradr", "k_gradz"):
         nf = Nfr if name == "k_gradr" else Nfz
         return nf * (q * wr + w) + N * (q * wr + 2 * w + 8)

@@ -47,7 +47,7 @@ DEFAULT_MB = (4, 6, 8, 10, 12, 16)
 # kernel name (as disco_batch_kernel_times reports it) -> macro
 MACROS = {"k_begin": "MB_BEGIN", "k_faces": "MB_FACES", "k_gradr": "MB_GRAD",
           "k_flux_r": "MB_FLUX", "k_update": "MB_UPDATE", "k_c2p": "MB_C2P"}
-# the MHD family: k_grad = k_gradr + k_gradz, k_flux = k_flux_r + k_flux_z
+# the MHD family: k_grad = k_gradr + k_gradz, k_flux = k_flux_r + k_flux_z (one launch in 3D)
 MACROS_MHD = {"k_begin": "MB_MHD_BEGIN", "k_grad": "MB_MHD_GRAD", "k_flux": "MB_MHD_FLUX",
               "k_update": "MB_MHD_UPDATE", "k_c2p": "MB_MHD_C2P"}
 FAMILIES = {"hydro": {"macros": MACROS, "header": TUNED, "workload": "ragged64"},
@@ -139,7 +139,7 @@ def _child(lib, workload, precision, reps):
         for name, ms in b.kernel_times(cap=128):
             tot[name] = tot.get(name, 0.0) + ms
         tot["k_grad"] = tot.get("k_grad", 0.0) + tot.get("k_gradr", 0.0) + tot.get("k_gradz", 0.0)
-        tot["k_flux"] = tot.get("k_flux_r", 0.0) + tot.get("k_flux_z", 0.0)
+        tot["k_flux"] = tot.get("k_flux", 0.0) + tot.get("k_flux_r", 0.0) + tot.get("k_flux_z", 0.0)
         for k, v in tot.items():
             per.setdefault(k, []).append(v)
     b.sync()
