@@ -764,7 +764,7 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
    v.dp = dupload(b, b->dparams);
    v.ds = dupload(b, dstate);
    b->d_ann_blk0 = dupload(b, b->ann_blk0); b->d_ann_nblk = dupload(b, b->ann_nblk);
-   size_t N = (size_t)cell, Qn = (size_t)b->Q*N, Qf = (size_t)b->Q*face;
+   const size_t N = (size_t)cell, Nt = tiled_n(N), Qn = b->Q*Nt, Qf = b->Q*tiled_n(face);
    size_t rs = precision == DISCO_PREC_MIXED ? sizeof(float) : sizeof(double);
    v.prim = (double *)dalloc_bytes(b, Qn*rs);
    v.gradp = (double *)dalloc_bytes(b, Qn*rs);
@@ -801,8 +801,8 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
       v.nfs = b->nfs;
       size_t ne = ct == 2 ? 8 : 4;
       auto ralloc = [&](size_t n){ return (double *)dalloc_bytes(b, n*rs); };   /* R-typed */
-      v.Phi = dalloc<double>(b, b->nfs*N); v.RKPhi = dalloc<double>(b, b->nfs*N);
-      v.ctE = ralloc(ne*N); v.ctB = ralloc(ne*N);
+      v.Phi = dalloc<double>(b, b->nfs*Nt); v.RKPhi = dalloc<double>(b, b->nfs*Nt);
+      v.ctE = ralloc(ne*Nt); v.ctB = ralloc(ne*Nt);
       v.pE = ralloc(N); v.pB = ralloc(N);
       v.fEt = ralloc(face); v.fBt = ralloc(face);
       v.fX = dalloc<double>(b, face);
@@ -941,13 +941,13 @@ template<class T>
 __global__ void k_aos_to_soa(const double *src, T *dst, size_t N, int Q){
    size_t c = blockIdx.x*(size_t)blockDim.x + threadIdx.x;
    if( c >= N ) return;
-   for( int q=0 ; q<Q ; ++q ) dst[q*N + c] = (T)src[c*Q + q];
+   for( int q=0 ; q<Q ; ++q ) dst[at_rows(Q, q, c)] = (T)src[c*Q + q];
 }
 template<class T>
 __global__ void k_soa_to_aos(const T *src, double *dst, size_t N, int Q){
    size_t c = blockIdx.x*(size_t)blockDim.x + threadIdx.x;
    if( c >= N ) return;
-   for( int q=0 ; q<Q ; ++q ) dst[c*Q + q] = (double)src[q*N + c];
+   for( int q=0 ; q<Q ; ++q ) dst[c*Q + q] = (double)src[at_rows(Q, q, c)];
 }
 static int staging(disco_batch *b){
    if( b->d_stage ) return DISCO_OK;
@@ -1004,7 +1004,7 @@ extern "C" int disco_batch_set_cells(disco_batch *b, const double *prim, const d
       if( Phi ){
          if( (s = upload_q<double>(b, b->vd.Phi, Phi, b->nfs)) ) return s;
       }else{
-         CK(cudaMemsetAsync(b->vd.Phi, 0, (size_t)b->nfs*N*sizeof(double), b->stream));
+         CK(cudaMemsetAsync(b->vd.Phi, 0, (size_t)b->nfs*tiled_n(N)*sizeof(double), b->stream));
       }
    }
    auto up = [&](double *dev, const double *src){
@@ -1013,7 +1013,7 @@ extern "C" int disco_batch_set_cells(disco_batch *b, const double *prim, const d
    CK(up(b->vd.piph, piph));
    CK(up(b->vd.dphi, dphi));
    if( wiph ) CK(up(b->vd.wiph, wiph));
-   if( b->vd.ccarry ) CK(cudaMemsetAsync(b->vd.ccarry, 0, (size_t)b->Q*N*sizeof(float), b->stream));
+   if( b->vd.ccarry ) CK(cudaMemsetAsync(b->vd.ccarry, 0, (size_t)b->Q*tiled_n(N)*sizeof(float), b->stream));
    b->topo_known = 0;
    CK(cudaMemsetAsync(b->vd.topo, 0, sizeof(int), b->stream));      /* new piph: faces stale */
    if( prim && !cons ){
@@ -1252,10 +1252,7 @@ extern "C" int disco_batch_restart_cells(disco_batch *b, const double *prim, con
    int s;
    if( (s = upload_r(b, b->vd.prim, prim)) ) return s;
    if( b->ct ){
-      const int F = b->nfs;
-      std::vector<double> t(F*N);
-      for( size_t c=0 ; c<N ; ++c ) for( int q=0 ; q<F ; ++q ) t[q*N + c] = Phi[F*c + q];
-      CK(xfer(b, b->vd.Phi, t.data(), t.size()*sizeof(double), cudaMemcpyHostToDevice));
+      if( (s = upload_q<double>(b, b->vd.Phi, Phi, b->nfs)) ) return s;
    }
    CK(xfer(b, b->vd.piph, piph, N*sizeof(double), cudaMemcpyHostToDevice));
    b->topo_known = 0;

@@ -63,9 +63,8 @@ __device__ __forceinline__ bool ct_phi_annulus(const DiskParams &P, int j, int k
 /* the slot holding face f's flux under its current LRtype (z: zf) */
 template<class R>
 __device__ __forceinline__ double *ct_slot(const ViewT<R> &v, double *base, int f, bool zf){
-   size_t N = v.Ncell;
-   if( zf ) return v.fLR[f] == 0 ? base + 4*N + v.fL[f] : base + 3*N + v.fR[f];
-   return v.fLR[f] == 0 ? base + 2*N + v.fL[f] : base + N + v.fR[f];
+   if( zf ) return v.fLR[f] == 0 ? base + AT_PHI(4, v.fL[f]) : base + AT_PHI(3, v.fR[f]);
+   return v.fLR[f] == 0 ? base + AT_PHI(2, v.fL[f]) : base + AT_PHI(1, v.fR[f]);
 }
 
 /* fn(f) for each face of cell i's runs in track t, in face order */
@@ -83,7 +82,6 @@ __global__ void __launch_bounds__(CB) k_ct_edges(ViewT<R> v){
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
    if( i >= np ) return;
-   const size_t N = v.Ncell;
    int c0 = b.c0, c = c0 + i;
    int cm = c0 + (i == 0 ? np-1 : i-1);
    const DiskParams &P = v.dp[b.disk];
@@ -135,7 +133,7 @@ __global__ void __launch_bounds__(CB) k_ct_edges(ViewT<R> v){
       }
    }
 #pragma unroll
-   for( int s=0 ; s<8 ; ++s ) if( s < ne ){ v.ctE[s*N + c] = E[s]; v.ctB[s*N + c] = B[s]; }
+   for( int s=0 ; s<8 ; ++s ) if( s < ne ){ v.ctE[AT_EDGE(s, c)] = E[s]; v.ctB[AT_EDGE(s, c)] = B[s]; }
 }
 
 /* next / previous cell of annulus a (cyclic) */
@@ -158,7 +156,6 @@ __global__ void __launch_bounds__(FB) k_ct_faces(ViewT<R> v){
    if( zf && v.ct != 2 ) return;
    int f = b.f0 + b.y + threadIdx.x;
    if( f >= b.f1 ) return;
-   const size_t N = v.Ncell;
    int A = b.A, Bn = b.B;
    int d = b.disk;
    const DiskParams &P = v.dp[d];
@@ -180,10 +177,10 @@ __global__ void __launch_bounds__(FB) k_ct_faces(ViewT<R> v){
    const R w1 = (R)dp1, w2 = (R)dp2;
    /* owner edge s_o (and its left twin s_o+2); c2's edges s_c, s_c+2 */
    size_t so = lr == 0 ? s0+1 : s0, sc = lr == 0 ? s0 : s0+1;
-   R Eo = R(.5)*(E[so*N + o] + E[(so+2)*N + on]);
-   R Bo = R(.5)*(B[so*N + o] + B[(so+2)*N + on]);
-   R ea = R(.5)*(E[sc*N + c2] + E[(sc+2)*N + c2n]), eb = R(.5)*(E[sc*N + c2p] + E[(sc+2)*N + c2]);
-   R ba = R(.5)*(B[sc*N + c2] + B[(sc+2)*N + c2n]), bb = R(.5)*(B[sc*N + c2p] + B[(sc+2)*N + c2]);
+   R Eo = R(.5)*(E[AT_EDGE(so, o)] + E[AT_EDGE(so+2, on)]);
+   R Bo = R(.5)*(B[AT_EDGE(so, o)] + B[AT_EDGE(so+2, on)]);
+   R ea = R(.5)*(E[AT_EDGE(sc, c2)] + E[AT_EDGE(sc+2, c2n)]), eb = R(.5)*(E[AT_EDGE(sc, c2p)] + E[AT_EDGE(sc+2, c2)]);
+   R ba = R(.5)*(B[AT_EDGE(sc, c2)] + B[AT_EDGE(sc+2, c2n)]), bb = R(.5)*(B[AT_EDGE(sc, c2p)] + B[AT_EDGE(sc+2, c2)]);
    R Eav = ( w2*ea + w1*eb )/(w1+w2);
    R Bav = ( w2*ba + w1*bb )/(w1+w2);
    R fE = R(.5)*(Eo + Eav);
@@ -451,7 +448,6 @@ __global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
    if( i >= np ) return;
-   const size_t N = v.Ncell;
    int c0 = b.c0, c = c0 + i;
    const DiskParams &P = v.dp[b.disk];
    int j = b.j, k = b.k;
@@ -462,8 +458,8 @@ __global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
    /* the RK snapshot / average of the slots (timestep.c:22, adjust_RK_cons
     * misc.c:239-241), taken here as their one read before the update */
    double st[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-   if( z3 ) rk_start<5>(v.Phi, v.RKPhi, N, c, first, st);
-   else     rk_start<3>(v.Phi, v.RKPhi, N, c, first, st);
+   if( z3 ) rk_start<5>(v.Phi, v.RKPhi, v.nfs, c, first, st);
+   else     rk_start<3>(v.Phi, v.RKPhi, v.nfs, c, first, st);
    double P0 = st[0], S1 = st[1], S2 = st[2], S3 = st[3], S4 = st[4];
    int f1 = -1, f2 = -1, f3 = -1, f4 = -1, t1 = 0, t2 = 0, t3 = 0, t4 = 0;
    if( j >= 1 ){                           /* inner r face: owned with LRtype 1 */
@@ -515,14 +511,14 @@ __global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
          if( j >= 1 )      S3 = ct_line_terms(v, S3, ln + (j-1) + W*(k-1), t3, f3, 0, 1.0);
          if( j <= P.Nr-2 ) S3 = ct_line_terms(v, S3, ln + j + W*(k-1), t3, f3, 1, -1.0);
       }
-      v.Phi[3*N + c] = S3;
-      v.Phi[4*N + c] = S4;
+      v.Phi[AT_PHI(3, c)] = S3;
+      v.Phi[AT_PHI(4, c)] = S4;
       if( !first && f3 >= 0 ) v.fPhi[f3] = S3;
       if( !first && f4 >= 0 ) v.fPhi[f4] = S4;
    }
-   v.Phi[N + c] = S1;
-   v.Phi[2*N + c] = S2;
-   v.Phi[c] = P0;
+   v.Phi[AT_PHI(1, c)] = S1;
+   v.Phi[AT_PHI(2, c)] = S2;
+   v.Phi[AT_PHI(0, c)] = P0;
    if( !first && f1 >= 0 ) v.fPhi[f1] = S1;
    if( !first && f2 >= 0 ) v.fPhi[f2] = S2;
    if( first ){
@@ -598,7 +594,6 @@ template<class R, bool FACE>
 __device__ void ct_cons_B(const ViewT<R> &v, const DiskParams &P, int a, int c0, int np, int i,
                           int j, int k, double rp, double rm, double zp, double zm, double *cons,
                           int *err){
-   const size_t N = v.Ncell;
    int c = c0 + i, cm = c0 + (i == 0 ? np-1 : i-1);
    int I0 = v.I0[a];
    double S = 0.0, T = 0.0;
@@ -621,10 +616,10 @@ __device__ void ct_cons_B(const ViewT<R> &v, const DiskParams &P, int a, int c0,
        * the cell's run in its inner (lower) track has the cell as R, in its
        * outer (upper) track as L; the other side's cell is read only when
        * that one owns the face */
-      auto sum_in = [&](int f){ S += v.fLR[f] == 0 ? v.Phi[2*N + v.fL[f]] : v.Phi[N + c]; T += v.fdA[f]; };
-      auto sum_out = [&](int f){ S += v.fLR[f] == 0 ? v.Phi[2*N + c] : v.Phi[N + v.fR[f]]; T += v.fdA[f]; };
-      auto sum_zin = [&](int f){ Sz += v.fLR[f] == 0 ? v.Phi[4*N + v.fL[f]] : v.Phi[3*N + c]; Tz += v.fdA[f]; };
-      auto sum_zout = [&](int f){ Sz += v.fLR[f] == 0 ? v.Phi[4*N + c] : v.Phi[3*N + v.fR[f]]; Tz += v.fdA[f]; };
+      auto sum_in = [&](int f){ S += v.fLR[f] == 0 ? v.Phi[AT_PHI(2, v.fL[f])] : v.Phi[AT_PHI(1, c)]; T += v.fdA[f]; };
+      auto sum_out = [&](int f){ S += v.fLR[f] == 0 ? v.Phi[AT_PHI(2, c)] : v.Phi[AT_PHI(1, v.fR[f])]; T += v.fdA[f]; };
+      auto sum_zin = [&](int f){ Sz += v.fLR[f] == 0 ? v.Phi[AT_PHI(4, v.fL[f])] : v.Phi[AT_PHI(3, c)]; Tz += v.fdA[f]; };
+      auto sum_zout = [&](int f){ Sz += v.fLR[f] == 0 ? v.Phi[AT_PHI(4, c)] : v.Phi[AT_PHI(3, v.fR[f])]; Tz += v.fdA[f]; };
       if( j >= 1 )      ct_over_runs(v, v.consR, tri, c0, np, i, I0, sum_in);
       if( j <= P.Nr-2 ) ct_over_runs(v, v.consL, tro, c0, np, i, I0, sum_out);
       if( z3 && k >= 1 )      ct_over_runs(v, v.consZR, tzi, c0, np, i, I0, sum_zin);
@@ -637,7 +632,7 @@ __device__ void ct_cons_B(const ViewT<R> &v, const DiskParams &P, int a, int c0,
    double rfac = 1.0/x0;                                /* bfield_scale_factor(x0, 0) */
    double hr = 1.0, hp = x0;
    cons[BRR] = S * (dV*rfac/(T * hr));
-   cons[BPP] = .5*(v.Phi[c]+v.Phi[cm])*dV/(dA * hp);
+   cons[BPP] = .5*(v.Phi[AT_PHI(0, c)]+v.Phi[AT_PHI(0, cm)])*dV/(dA * hp);
    if( z3 ){
       double zfac = 1.0, hz = 1.0;                      /* bfield_scale_factor(x2, 2) */
       cons[BZZ] = Sz * (dV*zfac/(Tz * hz));

@@ -8,7 +8,9 @@
  *                a Kahan-compensated FP64 conserved update.
  *
  * Layout (device, one batch of one or more disks):
- *   cells      ragged SoA in annulus order; prim[q*Ncell + c] (R), cons (FP64),
+ *   cells      ragged, in annulus order; an array of several fields in tiles of
+ *              TILE cells, a tile's fields one after another (at_rows):
+ *              prim (R), cons (FP64),
  *              RKcons (FP64), ccarry (FP32 Kahan carry, mixed form), gradp,
  *              gradr (R);
  *              piph[c], dphi[c], wiph[c] (FP64)
@@ -124,6 +126,27 @@ struct __align__(16) FaceBlk { int x, y;          /* track, first face within it
                                int A, B, NA, NB, cA0, cB0;   /* its annuli, their cells */
                                int disk, j, k, dim, flux, pad; };
 
+/* Element (q, c) of an array of L fields over the cells or faces: tiles of
+ * TILE cells, the fields of a tile one after another.  A warp's loads of a
+ * field are as consecutive as with each field in a row of its own, but all
+ * fields of a cell lie within a few kB instead of Ncell apart.  The step
+ * kernels wait on memory, and a gather over Q rows of hundreds of MB waits on
+ * address translation as well: ms per step, rows -> tiles, k_grad, k_faces
+ * and k_flux of 32 disks of the 3D binary (mixed) 2.187 -> 1.884, 2.511 ->
+ * 2.294 and 3.367 -> 3.007, the step 22.1 -> 20.6; 64 ragged disks FP64 4.288
+ * -> 4.117, GRMHD torus 6.262 -> 5.971, one small disk 0.178 -> 0.175.  Tiles
+ * of 128 are 0.2-0.4% slower; prim with its slopes, and cons with RKcons, in
+ * one array each 0.5% slower than apart. */
+#define TILE 32
+__host__ __device__ __forceinline__ size_t at_rows(int L, int q, unsigned c){
+   return (size_t)(c & ~(TILE-1u))*(L-1) + c + q*TILE;
+}
+static inline size_t tiled_n(size_t n){ return (n + TILE-1)/TILE*TILE; }
+/* of a state, of the face fluxes Phi and of the CT edge values of view v */
+#define AT(q, c) at_rows(Q, q, c)
+#define AT_PHI(s, c) at_rows(v.nfs, s, c)
+#define AT_EDGE(s, c) at_rows(v.ct == 2 ? 8 : 4, s, c)
+
 template<class R>
 struct ViewT {
    int Ncell, Nann, Ntr, Nf;
@@ -172,8 +195,8 @@ struct ViewT {
    double dtfac;        /* 1 in the first substep, 0.5 in the second (timestep.c:39) */
    int *err;
    /* Constrained transport (Constrained_Transport 1; bfields.c), ct = the
-    * CT_MODE (1: 2D, NUM_FACES 3; 2: 3D, NUM_FACES 5) or 0.  Per cell, SoA
-    * [s*Ncell + c]: Phi / RKPhi, s = 0 the magnetic flux through the cell's
+    * CT_MODE (1: 2D, NUM_FACES 3; 2: 3D, NUM_FACES 5) or 0.  Per cell
+    * [AT_PHI(s, c)]: Phi / RKPhi, s = 0 the magnetic flux through the cell's
     * phi face at piph, s = 1 / 2 the flux through the r-face the cell owns in
     * the track inside / outside it (the face ending at its piph, LRtype 1 /
     * 0), s = 3 / 4 the same for the z-faces below / above it; ctE / ctB the
@@ -247,12 +270,11 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid
    const CellBlk b = v.cblk[bid];
    int a = b.x, i0 = b.y, t = threadIdx.x, i = i0 + t;
    int np = b.np;
-   const int N = v.Ncell;
    int c0 = b.c0, c = c0 + i;
    int nact = np - i0 < CB ? np - i0 : CB;
    auto stage = [&](int slot, int cell){
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) sp[q][slot] = v.prim[q*N + cell];
+      for( int q=0 ; q<Q ; ++q ) sp[q][slot] = v.prim[AT(q, cell)];
       sd[slot] = v.dphi[cell];
    };
    if( t < nact ) stage(t+1, c);
@@ -314,7 +336,7 @@ __device__ __forceinline__ void begin_body(const ViewT<R> &v, int first, int bid
       if( fabs(bb) < fabs(m) ) m = bb;
       if( bb*cc < R(0.0) ) m = R(0.0);
       if( fabs(cc) < fabs(m) ) m = cc;
-      v.gradp[q*N + c] = m;
+      v.gradp[AT(q, c)] = m;
    }
 }
 /* Energy-frame Omega at the radii the step evaluates it (omega.c:62-110):
@@ -502,10 +524,9 @@ __device__ __forceinline__ int gallop_lb(int lo, int hi, int g, Pr p){
  * (0.782 field by field, 0.911 together, 1.014 together at 10 blocks). */
 template<int Q, class R>
 __device__ __forceinline__ void face_slopes(const ViewT<R> &v, int cL, int cR, R dpL, R dpR, R dxL, R dxR, int f){
-   const int N = v.Ncell;
    auto slope = [&](int q){
-      R WL = v.prim[q*N + cL] + dpL*v.gradp[q*N + cL];
-      R WR = v.prim[q*N + cR] - dpR*v.gradp[q*N + cR];
+      R WL = v.prim[AT(q, cL)] + dpL*v.gradp[AT(q, cL)];
+      R WR = v.prim[AT(q, cR)] - dpR*v.gradp[AT(q, cR)];
       return (WR-WL)/(dxR+dxL);
    };
    if constexpr ( sizeof(R) == sizeof(float) ){
@@ -513,10 +534,10 @@ __device__ __forceinline__ void face_slopes(const ViewT<R> &v, int cL, int cR, R
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ) S[q] = slope(q);
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) v.fS[(size_t)q*v.Nf + f] = S[q];
+      for( int q=0 ; q<Q ; ++q ) v.fS[AT(q, f)] = S[q];
    }else{
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) v.fS[(size_t)q*v.Nf + f] = slope(q);
+      for( int q=0 ; q<Q ; ++q ) v.fS[AT(q, f)] = slope(q);
    }
 }
 
@@ -527,7 +548,6 @@ __device__ __forceinline__ void faces_body(const ViewT<R> &v, int with_slopes, i
    int A = b.A, B = b.B;
    int NA = b.NA, NB = b.NB;
    if( dd >= NA + NB ) return;
-   const int N = v.Ncell;
    int f = b.f0 + dd;
    int cA0 = b.cA0, cB0 = b.cB0;
    int IA = v.I0[A], IB = v.I0[B];
@@ -650,7 +670,6 @@ __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
    if( i >= np ) return;
-   const int N = v.Ncell;
    int c0 = b.c0, c = c0 + i;
    int d = b.disk;
    const DiskParams &P = v.dp[d];
@@ -664,7 +683,7 @@ __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
    for( int q=0 ; q<Q ; ++q ) g[q] = R(0.0);
    if( P.PLM == 0.0 ){
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) grad[q*N + c] = R(0.0);
+      for( int q=0 ; q<Q ; ++q ) grad[AT(q, c)] = R(0.0);
       return;
    }
    int tin, tout;
@@ -683,7 +702,7 @@ __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
    if( tout >= 0 ) Rout = cell_runs(v, cout, tout, c0, np, i, I0);
    const size_t Nf = v.Nf;
 #define ACC_RUN(s,e) for( int f=(s) ; f<=(e) ; ++f ){ R dA = (R)v.fdA[f]; \
-      _Pragma("unroll") for( int q=0 ; q<Q ; ++q ) g[q] += v.fS[q*Nf + f]*dA; }
+      _Pragma("unroll") for( int q=0 ; q<Q ; ++q ) g[q] += v.fS[AT(q, f)]*dA; }
    ACC_RUN(Rin.s1, Rin.e1)
    ACC_RUN(Rin.s2, Rin.e2)
    ACC_RUN(Rout.s1, Rout.e1)
@@ -713,7 +732,7 @@ __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
    for( int q=0 ; q<Q ; ++q ) g[q] /= rdAtot;
    const R PLM = (R)P.PLM;
 #define LIM_RUN(s,e) for( int f=(s) ; f<=(e) ; ++f ){ \
-      _Pragma("unroll") for( int q=0 ; q<Q ; ++q ){ R S = v.fS[q*Nf + f]; \
+      _Pragma("unroll") for( int q=0 ; q<Q ; ++q ){ R S = v.fS[AT(q, f)]; \
          if( S*g[q] < R(0.0) ) g[q] = R(0.0); else if( fabs(PLM*S) < fabs(g[q]) ) g[q] = PLM*S; } }
    LIM_RUN(Rin.s1, Rin.e1)
    LIM_RUN(Rin.s2, Rin.e2)
@@ -732,7 +751,7 @@ __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
 #pragma unroll
          for( int q=0 ; q<Q ; ++q ){
             if( q == URR || (Q > 6 && q == BRR) ){
-               double SL = (double)v.prim[q*N + c]/r;
+               double SL = (double)v.prim[AT(q, c)]/r;
                double S = (double)g[q];
                if( S*SL < 0.0 ) g[q] = R(0.0);
                else if( fabs(P.PLM*SL) < fabs(S) ) g[q] = (R)(P.PLM*SL);
@@ -743,7 +762,7 @@ __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
       }
    }
 #pragma unroll
-   for( int q=0 ; q<Q ; ++q ) grad[q*N + c] = g[q];
+   for( int q=0 ; q<Q ; ++q ) grad[AT(q, c)] = g[q];
    raise_err(v, err);
 }
 /* The r direction, with D3 also the z direction of a 3D grid (the cell's
@@ -768,18 +787,17 @@ template<int Q, int DIM, class R>
 __device__ __forceinline__ void trans_visc_flux(const ViewT<R> &v, const DiskParams &P, int cL, int cR,
                                              R dpL, R dpR, R dxL, R dxR, const R *primL,
                                              const R *primR, double r, double om, double *vF){
-   const int N = v.Ncell;
    double pa[Q], gr[Q], gp[Q], gz[Q];
    for( int q=0 ; q<Q ; ++q ){
-      double g = (((double)v.prim[q*N+cR] - (double)v.gradp[q*N+cR]*(double)dpR)
-                  - ((double)v.prim[q*N+cL] + (double)v.gradp[q*N+cL]*(double)dpL))
+      double g = (((double)v.prim[AT(q, cR)] - (double)v.gradp[AT(q, cR)]*(double)dpR)
+                  - ((double)v.prim[AT(q, cL)] + (double)v.gradp[AT(q, cL)]*(double)dpL))
                  / ((double)dxL + (double)dxR);
-      double zL = v.gradz ? (double)v.gradz[q*N+cL] : 0.0;
-      double zR = v.gradz ? (double)v.gradz[q*N+cR] : 0.0;
+      double zL = v.gradz ? (double)v.gradz[AT(q, cL)] : 0.0;
+      double zR = v.gradz ? (double)v.gradz[AT(q, cR)] : 0.0;
       pa[q] = .5*((double)primL[q] + (double)primR[q]);
-      gp[q] = .5*((double)v.gradp[q*N+cL] + (double)v.gradp[q*N+cR]);
+      gp[q] = .5*((double)v.gradp[AT(q, cL)] + (double)v.gradp[AT(q, cR)]);
       if( DIM == 1 ){ gr[q] = .5*(g + g); gz[q] = .5*(zL + zR); }
-      else { gr[q] = .5*((double)v.gradr[q*N+cL] + (double)v.gradr[q*N+cR]); gz[q] = .5*(g + g); }
+      else { gr[q] = .5*((double)v.gradr[AT(q, cL)] + (double)v.gradr[AT(q, cR)]); gz[q] = .5*(g + g); }
    }
    const double n[3] = {DIM == 1 ? 1.0 : 0.0, 0.0, DIM == 2 ? 1.0 : 0.0};
    visc_flux<Q>(P, pa, gr, gp, gz, r, om, n, vF);
@@ -788,15 +806,14 @@ template<int Q, class R>
 __device__ __forceinline__ void phi_visc_flux(const ViewT<R> &v, const DiskParams &P, int cL, int cR,
                                            const R *primL, const R *primR, double r, double om,
                                            double *vF){
-   const int N = v.Ncell;
    double pa[Q], gr[Q], gp[Q], gz[Q];
    double dh = 0.5*(v.dphi[cR] + v.dphi[cL]);
    for( int q=0 ; q<Q ; ++q ){
-      double g = ((double)v.prim[q*N+cR] - (double)v.prim[q*N+cL]) / dh;
+      double g = ((double)v.prim[AT(q, cR)] - (double)v.prim[AT(q, cL)]) / dh;
       pa[q] = .5*((double)primL[q] + (double)primR[q]);
-      gr[q] = .5*((double)v.gradr[q*N+cL] + (double)v.gradr[q*N+cR]);
+      gr[q] = .5*((double)v.gradr[AT(q, cL)] + (double)v.gradr[AT(q, cR)]);
       gp[q] = .5*(g + g);
-      gz[q] = v.gradz ? .5*((double)v.gradz[q*N+cL] + (double)v.gradz[q*N+cR]) : 0.0;
+      gz[q] = v.gradz ? .5*((double)v.gradz[AT(q, cL)] + (double)v.gradz[AT(q, cR)]) : 0.0;
    }
    const double n[3] = {0.0, 1.0, 0.0};
    visc_flux<Q>(P, pa, gr, gp, gz, r, om, n, vF);
@@ -816,13 +833,12 @@ __device__ __forceinline__ void trans_face_flux_visc(const ViewT<R> &v, const Di
 template<int Q, class R>
 __device__ __forceinline__ double2 visc_source_cell(const ViewT<R> &v, const DiskParams &P, int c,
                                                  int a, double r, double dVdt){
-   const int N = v.Ncell;
    double gr[Q], gp[Q], gz[Q], prim[Q];
-   for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[q*N + c];
+   for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[AT(q, c)];
    for( int q=0 ; q<Q ; ++q ){
-      gr[q] = (double)v.gradr[q*N + c];
-      gp[q] = (double)v.gradp[q*N + c];
-      gz[q] = v.gradz ? (double)v.gradz[q*N + c] : 0.0;
+      gr[q] = (double)v.gradr[AT(q, c)];
+      gp[q] = (double)v.gradp[AT(q, c)];
+      gz[q] = v.gradz ? (double)v.gradz[AT(q, c)] : 0.0;
    }
    double nu = visc_nu(P, prim, r);
    double rho = prim[RHO], vr = prim[URR];
@@ -850,7 +866,6 @@ __device__ __forceinline__ void flux_body(const ViewT<R> &v, double dtfac, int b
    int dd = b.y + threadIdx.x;
    int f = b.f0 + dd;
    if( f >= b.f1 ) return;
-   const int N = v.Ncell;
    int cL = v.fL[f], cR = v.fR[f];
    int d = b.disk;
    const DiskParams &P = v.dp[d];
@@ -867,8 +882,8 @@ __device__ __forceinline__ void flux_body(const ViewT<R> &v, double dtfac, int b
    R primL[Q], primR[Q];
 #pragma unroll
    for( int q=0 ; q<Q ; ++q ){
-      primL[q] = v.prim[q*N+cL] + grad[q*N+cL]*dxL + v.gradp[q*N+cL]*dpL;
-      primR[q] = v.prim[q*N+cR] - grad[q*N+cR]*dxR - v.gradp[q*N+cR]*dpR;
+      primL[q] = v.prim[AT(q, cL)] + grad[AT(q, cL)]*dxL + v.gradp[AT(q, cL)]*dpL;
+      primR[q] = v.prim[AT(q, cR)] - grad[AT(q, cR)]*dxR - v.gradp[AT(q, cR)]*dpR;
    }
    if constexpr ( NC == 8 ){                     /* normal B averaged, riemann.c:146-152 */
       const int BT = DIM == 1 ? BRR : BZZ;
@@ -919,7 +934,7 @@ __device__ __forceinline__ void flux_body(const ViewT<R> &v, double dtfac, int b
       }
    }
 #pragma unroll
-   for( int q=0 ; q<Q ; ++q ) v.fG[(size_t)q*v.Nf + f] = G[q];
+   for( int q=0 ; q<Q ; ++q ) v.fG[AT(q, f)] = G[q];
    raise_err(v, err);
 }
 /* the blocks of v.fblk: DIRS 1 of r tracks, 2 of z tracks, 3 the first nr
@@ -939,13 +954,12 @@ template<int Q, int NC, class R>
 __device__ __forceinline__ void phi_face_flux(const ViewT<R> &v, const DiskParams &P, int a,
                                               int cL, int cR, double r, double dAdt, R *G,
                                               R *eb = nullptr){
-   const int N = v.Ncell;
    R primL[Q], primR[Q];
    R dL = (R)v.dphi[cL], dR = (R)v.dphi[cR];
 #pragma unroll
    for( int q=0 ; q<Q ; ++q ){
-      primL[q] = v.prim[q*N+cL] + R(.5)*v.gradp[q*N+cL]*dL;
-      primR[q] = v.prim[q*N+cR] - R(.5)*v.gradp[q*N+cR]*dR;
+      primL[q] = v.prim[AT(q, cL)] + R(.5)*v.gradp[AT(q, cL)]*dL;
+      primR[q] = v.prim[AT(q, cR)] - R(.5)*v.gradp[AT(q, cR)]*dR;
    }
    if constexpr ( NC == 8 ){                     /* B_phi averaged, riemann.c:54-58 */
       R Bp = R(.5)*(primL[BPP]+primR[BPP]);
@@ -983,12 +997,11 @@ template<int Q, class R> struct QVec { R q[Q]; };
 template<int Q, int NC, class R>
 __device__ __forceinline__ QVec<Q,R> phi_face_flux_visc(const ViewT<R> &v, const DiskParams &P, int a,
                                                      int cL, int cR, double r, double dAdt){
-   const int N = v.Ncell;
    R primL[Q], primR[Q];
    R dL = (R)v.dphi[cL], dR = (R)v.dphi[cR];
    for( int q=0 ; q<Q ; ++q ){
-      primL[q] = v.prim[q*N + cL] + R(.5)*v.gradp[q*N + cL]*dL;
-      primR[q] = v.prim[q*N + cR] - R(.5)*v.gradp[q*N + cR]*dR;
+      primL[q] = v.prim[AT(q, cL)] + R(.5)*v.gradp[AT(q, cL)]*dL;
+      primR[q] = v.prim[AT(q, cR)] - R(.5)*v.gradp[AT(q, cR)]*dR;
    }
    double w = r*v.wiph[cL];
    double vF[Q];
@@ -1006,18 +1019,18 @@ __device__ __forceinline__ QVec<Q,R> phi_face_flux_visc(const ViewT<R> &v, const
  * step, 64 disks 1.031 -> 0.996 (mixed 1.009 -> 0.940), MHD 64x64 annuli
  * 0.637 -> 0.599; k_ct_update of 32 disks of binary_nz 2.147 -> 1.870. */
 template<int M>
-__device__ __forceinline__ void rk_start(const double *x, double *RKx, size_t N, size_t c, int first, double *x0){
+__device__ __forceinline__ void rk_start(const double *x, double *RKx, int L, int c, int first, double *x0){
 #pragma unroll
-   for( int q=0 ; q<M ; ++q ) x0[q] = x[q*N + c];
+   for( int q=0 ; q<M ; ++q ) x0[q] = x[at_rows(L, q, c)];
    if( first ){
 #pragma unroll
       for( int q=0 ; q<M ; ++q ){
-         RKx[q*N + c] = x0[q];
+         RKx[at_rows(L, q, c)] = x0[q];
          if( !isfinite(x0[q]) ) x0[q] = x0[q] + 0.0*x0[q];
       }
    }else{
 #pragma unroll
-      for( int q=0 ; q<M ; ++q ) x0[q] = (1.-.5)*x0[q] + .5*RKx[q*N + c];
+      for( int q=0 ; q<M ; ++q ) x0[q] = (1.-.5)*x0[q] + .5*RKx[at_rows(L, q, c)];
    }
 }
 
@@ -1047,7 +1060,6 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
    const CellBlk b = v.ublk[bid];
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
-   const int N = v.Ncell;
    int c0 = b.c0, c = c0 + i;
    int cprev = c0 + (i == 0 ? np-1 : i-1);
    int d = b.disk;
@@ -1071,9 +1083,9 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       /* what the gather reads after the phi faces, on its way to L2 meanwhile */
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ){
-         prefetch_l2(v.cons + (size_t)q*N + c);
-         if( !first ) prefetch_l2(v.RKcons + (size_t)q*N + c);
-         if constexpr ( sizeof(R) != sizeof(double) ) prefetch_l2(v.ccarry + (size_t)q*N + c);
+         prefetch_l2(v.cons + AT(q, c));
+         if( !first ) prefetch_l2(v.RKcons + AT(q, c));
+         if constexpr ( sizeof(R) != sizeof(double) ) prefetch_l2(v.ccarry + AT(q, c));
       }
       prefetch_l2(v.consL + c); prefetch_l2(v.consR + c);
       if( P.Nz > 1 ){ prefetch_l2(v.consZL + c); prefetch_l2(v.consZR + c); }
@@ -1091,7 +1103,7 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
          R dph = (R)v.dphi[cell];
 #pragma unroll
          for( int q=0 ; q<Q ; ++q ){
-            R pq = v.prim[q*N + cell], gq = v.gradp[q*N + cell];
+            R pq = v.prim[AT(q, cell)], gq = v.gradp[AT(q, cell)];
             if( right ) right[q] = pq + R(.5)*gq*dph;
             sW[q][slot] = pq - R(.5)*gq*dph;
          }
@@ -1160,11 +1172,11 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       for( int q=0 ; q<Q ; ++q ){
          if constexpr ( sizeof(R) != sizeof(double) ){
             /* the carry belongs to cons; averaged with it (RKcons keeps none) */
-            cc[q] = (double)v.ccarry[q*N + c];
+            cc[q] = (double)v.ccarry[AT(q, c)];
             if( !first ) cc[q] = (double)(float)(.5*cc[q]);
          }else cc[q] = 0.0;
       }
-      rk_start<Q>(v.cons, v.RKcons, N, c, first, cons);
+      rk_start<Q>(v.cons, v.RKcons, Q, c, first, cons);
       /* The face fluxes: in the FP64 path added to cons one by one in the
        * reference's order; in the mixed form (FP32 fluxes) summed in a plain
        * FP64 accumulator, exact for a handful of FP32 values whose exponents
@@ -1200,7 +1212,7 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       if( j <= P.Nr-2 ) Rout = cell_runs(v, v.consL, P.trr0 + j + (P.Nr-1)*k, c0, np, i, I0);
       const size_t Nf = v.Nf;
 #define ADD_RUN(s,e,sg) for( int f=(s) ; f<=(e) ; ++f ){ \
-      _Pragma("unroll") for( int q=0 ; q<Q ; ++q ) addf(q, sg (double)v.fG[q*Nf + f]); }
+      _Pragma("unroll") for( int q=0 ; q<Q ; ++q ) addf(q, sg (double)v.fG[AT(q, f)]); }
       ADD_RUN(Rin.s1, Rin.e1, +)
       ADD_RUN(Rin.s2, Rin.e2, +)
       ADD_RUN(Rout.s1, Rout.e1, -)
@@ -1226,7 +1238,7 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       /* add_source with the pre-move cell */
       double prim[Q];
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[q*N + c];
+      for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[AT(q, c)];
       double rp = rj[j], rm = rj[j-1], zp = zk[k], zm = zk[k-1];
       double phim = piph - dphi;
       double dph = get_dp(piph, phim, P.Pmax, &err);
@@ -1290,13 +1302,13 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       }
 #pragma unroll
       for( int q=0 ; q<Q ; ++q ){
-         v.cons[q*N + c] = cons[q];
-         if constexpr ( sizeof(R) != sizeof(double) ) v.ccarry[q*N + c] = (float)cc[q];
+         v.cons[AT(q, c)] = cons[q];
+         if constexpr ( sizeof(R) != sizeof(double) ) v.ccarry[AT(q, c)] = (float)cc[q];
       }
    }
    else if( first ){                /* a ghost's cons is not evolved: its snapshot alone */
       double x0[Q];
-      rk_start<Q>(v.cons, v.RKcons, N, c, first, x0);
+      rk_start<Q>(v.cons, v.RKcons, Q, c, first, x0);
    }
    /* the move follows in k_c2p (or k_ct_update) */
    raise_err(v, err);
@@ -1376,7 +1388,6 @@ __global__ void __launch_bounds__(CB) k_diag_part(ViewT<R> v){
    const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
-   const int N = v.Ncell;
    int d = b.disk;
    const DiskParams &P = v.dp[d];
    int j = b.j, k = b.k;
@@ -1390,7 +1401,7 @@ __global__ void __launch_bounds__(CB) k_diag_part(ViewT<R> v){
       int c = b.c0 + i;
       double prim[Q];
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[q*N + c];
+      for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[AT(q, c)];
       double piph = v.piph[c];
       diag_cell<NQD>(P, v.ds[d], prim, rj[j], rj[j-1], zk[k], zk[k-1], piph, piph - v.dphi[c], dq, &err);
    }
@@ -1596,7 +1607,7 @@ __device__ __forceinline__ void c2p_tail(const ViewT<R> &v, const DiskParams &P,
          double dV2 = dV_of(rp, rm, dph2, zp, zm);
          if constexpr ( GR ){       /* grmhd2 cons2prim from the cell's current prims */
 #pragma unroll
-            for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[q*N + c];
+            for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[AT(q, c)];
             double x[3] = {centroid_r(rp, rm), 0.5*(phim+piph), centroid_z(zp, zm)};
             if( v.gr_dump ){         /* the solve's inputs, as gr_cons2prim forms them */
                double *o = v.gr_dump + c;
@@ -1620,7 +1631,7 @@ __device__ __forceinline__ void c2p_tail(const ViewT<R> &v, const DiskParams &P,
 #pragma unroll
          for( int q=0 ; q<Q ; ++q ){
             R pq = (R)prim[q];
-            v.prim[q*N + c] = pq;
+            v.prim[AT(q, c)] = pq;
             prim[q] = (double)pq;       /* the stored state is what the next step sees */
          }
       }else{
@@ -1628,12 +1639,12 @@ __device__ __forceinline__ void c2p_tail(const ViewT<R> &v, const DiskParams &P,
 #pragma unroll
             for( int q=0 ; q<Q ; ++q ){
                R pq = (R)prim[q];
-               v.prim[q*N + c] = pq;
+               v.prim[AT(q, c)] = pq;
                prim[q] = (double)pq;
             }
          }else if( last ){
 #pragma unroll
-            for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[q*N + c];
+            for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[AT(q, c)];
          }
       }
       if( last ){
@@ -1717,7 +1728,6 @@ __device__ __forceinline__ void c2p_body(const ViewT<R> &v, int last, int bc, in
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
    bool active = i < np;
-   const int N = v.Ncell;
    int c0 = b.c0, c = c0 + (active ? i : 0);
    int d = b.disk;
    const DiskParams &P = v.dp[d];
@@ -1736,15 +1746,15 @@ __device__ __forceinline__ void c2p_body(const ViewT<R> &v, int last, int bc, in
       }
       if( real ){
 #pragma unroll
-         for( int q=0 ; q<Q ; ++q ) cons[q] = v.cons[q*N + c];
+         for( int q=0 ; q<Q ; ++q ) cons[q] = v.cons[AT(q, c)];
          if constexpr ( NC == 8 ){
             if( v.ct ){                  /* onestep.c:183-185 */
                const double *rj = v.rj + P.rj0 + 1;
                const double *zk = v.zk + P.zk0 + 1;
                ct_cons_B<R,FACE>(v, P, a, c0, np, i, j, k, rj[j], rj[j-1], zk[k], zk[k-1], cons, &err);
-               v.cons[BRR*N + c] = cons[BRR];
-               v.cons[BPP*N + c] = cons[BPP];
-               if( v.ct == 2 && P.Nz > 1 ) v.cons[BZZ*N + c] = cons[BZZ];
+               v.cons[AT(BRR, c)] = cons[BRR];
+               v.cons[AT(BPP, c)] = cons[BPP];
+               if( v.ct == 2 && P.Nz > 1 ) v.cons[AT(BZZ, c)] = cons[BZZ];
             }
          }
       }
@@ -1832,7 +1842,6 @@ __device__ __forceinline__ void zerograd_pair(const ViewT<R> &v, int2 pr, int sf
       const int j = v.ann_j[a], k = v.ann_k[a];
       const double *rj = v.rj + P.rj0 + 1;
       const double *zk = v.zk + P.zk0 + 1;
-      const int N = v.Ncell;
       for( int i=threadIdx.x ; i<np ; i+=blockDim.x ){
          const double phip = v.piph[c0+i], dp = v.dphi[c0+i];
          double phi = phip - 0.5*dp;
@@ -1843,7 +1852,7 @@ __device__ __forceinline__ void zerograd_pair(const ViewT<R> &v, int2 pr, int sf
             initial<Q, (Q > 6 ? 8 : 5)>(P, tp, x);
             if( P.rotframe ) tp[UPP] -= P.RotOmega;
 #pragma unroll
-            for( int q=0 ; q<Q ; ++q ) v.prim[q*N + c0 + i] = (R)tp[q];
+            for( int q=0 ; q<Q ; ++q ) v.prim[AT(q, c0 + i)] = (R)tp[q];
          }
       }
       return;
@@ -1930,7 +1939,6 @@ __device__ __forceinline__ void zerograd_pair(const ViewT<R> &v, int2 pr, int sf
       }
       __syncthreads();
    }
-   const int N = v.Ncell;
    for( int i=threadIdx.x ; i<np ; i+=blockDim.x ){
       double phip = sp[i], phim = sp[i] - sd[i];
       double acc[Q];
@@ -1947,7 +1955,7 @@ __device__ __forceinline__ void zerograd_pair(const ViewT<R> &v, int2 pr, int sf
          double phi2 = phim > phim1 ? phim : phim1;
          double dphi = phi1 - phi2;
 #pragma unroll
-         for( int q=0 ; q<Q ; ++q ) acc[q] += (double)v.prim[q*N + c10 + i1]*dphi;
+         for( int q=0 ; q<Q ; ++q ) acc[q] += (double)v.prim[AT(q, c10 + i1)]*dphi;
          i1 = i1 < np1-1 ? i1+1 : 0;
       }
 #pragma unroll
@@ -1979,7 +1987,7 @@ __device__ __forceinline__ void zerograd_pair(const ViewT<R> &v, int2 pr, int sf
          out[UPP] = (R)tp[UPP];
       }
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) v.prim[q*N + c0 + i] = out[q];
+      for( int q=0 ; q<Q ; ++q ) v.prim[AT(q, c0 + i)] = out[q];
    }
 }
 template<int Q, class R>
@@ -2133,7 +2141,6 @@ __global__ void __launch_bounds__(CB) k_report_part(ViewT<R> v, double *part){
    const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
-   const int N = v.Ncell;
    int d = b.disk;
    const DiskParams &P = v.dp[d];
    const DiskState &S = v.ds[d];
@@ -2153,8 +2160,8 @@ __global__ void __launch_bounds__(CB) k_report_part(ViewT<R> v, double *part){
       double phim = phip - dphi;
       double dV = dV_of(rj[j], rj[j-1], get_dp(phip, phim, P.Pmax, &err), zk[k], zk[k-1]);
       double r = centroid_r(rj[j], rj[j-1]);
-      double rho = (double)v.prim[RHO*N + c], Pp = (double)v.prim[PPP*N + c];
-      double vr = (double)v.prim[URR*N + c];
+      double rho = (double)v.prim[AT(RHO, c)], Pp = (double)v.prim[AT(PPP, c)];
+      double vr = (double)v.prim[AT(URR, c)];
       double sn, cs;
       sincos(phi, &sn, &cs);
       const double rho0 = 1.0;
@@ -2164,8 +2171,8 @@ __global__ void __launch_bounds__(CB) k_report_part(ViewT<R> v, double *part){
       x[RP_L1RHO] = fabs(rho/rho0-1.)*dV;
       x[RP_L1P] = fabs(Pp/pow(rho, 5./3.)/0.01-1.)*dV;
       if constexpr ( NC == 8 ){
-         double Br = (double)v.prim[BRR*N + c], Bp = (double)v.prim[BPP*N + c];
-         double Bz = (double)v.prim[BZZ*N + c];
+         double Br = (double)v.prim[AT(BRR, c)], Bp = (double)v.prim[AT(BPP, c)];
+         double Bz = (double)v.prim[AT(BZZ, c)];
          x[RP_L1B] = fabs(Br)*dV;
          x[RP_BR2] = .5*Br*Br*dV;
          x[RP_BRBP] = Br*Bp*dV;
@@ -2265,7 +2272,6 @@ __global__ void __launch_bounds__(CB) k_setup(ViewT<R> v, int bc){
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
    if( i >= np ) return;
-   const int N = v.Ncell;
    int c = b.c0 + i;
    int d = b.disk;
    const DiskParams &P = v.dp[d];
@@ -2314,18 +2320,18 @@ __global__ void __launch_bounds__(CB) k_setup(ViewT<R> v, int bc){
          if( v.xflag ) v.xflag[c] = ex ? 1 : 0;
       }
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ){ v.prim[q*N+c] = (R)prim[q]; v.cons[q*N+c] = cons[q]; }
+      for( int q=0 ; q<Q ; ++q ){ v.prim[AT(q, c)] = (R)prim[q]; v.cons[AT(q, c)] = cons[q]; }
    }else{
       if( fixed_ghost_init<Q,NC>(P, bc, j, k, rj, zk, piph, dphi, prim) ){
 #pragma unroll
-         for( int q=0 ; q<Q ; ++q ) v.prim[q*N+c] = (R)prim[q];
+         for( int q=0 ; q<Q ; ++q ) v.prim[AT(q, c)] = (R)prim[q];
       }
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) v.cons[q*N+c] = 0.0;
+      for( int q=0 ; q<Q ; ++q ) v.cons[AT(q, c)] = 0.0;
    }
    if constexpr ( sizeof(R) != sizeof(double) ){
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) v.ccarry[q*N+c] = 0.0f;
+      for( int q=0 ; q<Q ; ++q ) v.ccarry[AT(q, c)] = 0.0f;
    }
    if constexpr ( NC == 8 ){
       if( v.ct ){                        /* set_B_fields, bfields.c:22-42 */
@@ -2333,8 +2339,8 @@ __global__ void __launch_bounds__(CB) k_setup(ViewT<R> v, int bc){
          double pb[Q];
          initial<Q,NC>(P, pb, x);
          double dA = (rj[j]-rj[j-1])*(zk[k]-zk[k-1]);
-         v.Phi[c] = pb[BPP]*dA;
-         for( int s=1 ; s<v.nfs ; ++s ) v.Phi[(size_t)s*N + c] = 0.0;
+         v.Phi[AT_PHI(0, c)] = pb[BPP]*dA;
+         for( int s=1 ; s<v.nfs ; ++s ) v.Phi[AT_PHI(s, c)] = 0.0;
       }
    }
    raise_err(v, err);
@@ -2353,7 +2359,6 @@ __global__ void __launch_bounds__(CB) k_restart(ViewT<R> v, int bc){
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
    if( i >= np ) return;
-   const int N = v.Ncell;
    int c0 = b.c0, c = c0 + i;
    int d = b.disk;
    const DiskParams &P = v.dp[d];
@@ -2373,7 +2378,7 @@ __global__ void __launch_bounds__(CB) k_restart(ViewT<R> v, int bc){
       double dph = get_dp(piph, piph - dphi, P.Pmax, &err);
       double dV = dV_of(rj[j], rj[j-1], dph, zk[k], zk[k-1]);
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[q*N+c];
+      for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[AT(q, c)];
       if( P.noise_type && v.noise ){                  /* domain.c:202-203, restart too */
          double x[3] = {r, piph - .5*dphi, z};
          add_noise(P.noise_type, P.noise_abs, P.noise_rel, prim, x, v.noise + 4*(size_t)c);
@@ -2401,18 +2406,18 @@ __global__ void __launch_bounds__(CB) k_restart(ViewT<R> v, int bc){
          if( v.xflag ) v.xflag[c] = ex ? 1 : 0;     /* setupCells marks the real cells anew */
       }
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ){ v.prim[q*N+c] = (R)prim[q]; v.cons[q*N+c] = cons[q]; }
+      for( int q=0 ; q<Q ; ++q ){ v.prim[AT(q, c)] = (R)prim[q]; v.cons[AT(q, c)] = cons[q]; }
    }else{
       if( fixed_ghost_init<Q,NC>(P, bc, j, k, rj, zk, piph, dphi, prim) ){
 #pragma unroll
-         for( int q=0 ; q<Q ; ++q ) v.prim[q*N+c] = (R)prim[q];
+         for( int q=0 ; q<Q ; ++q ) v.prim[AT(q, c)] = (R)prim[q];
       }
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) v.cons[q*N+c] = 0.0;
+      for( int q=0 ; q<Q ; ++q ) v.cons[AT(q, c)] = 0.0;
    }
    if constexpr ( sizeof(R) != sizeof(double) ){
 #pragma unroll
-      for( int q=0 ; q<Q ; ++q ) v.ccarry[q*N+c] = 0.0f;
+      for( int q=0 ; q<Q ; ++q ) v.ccarry[AT(q, c)] = 0.0f;
    }
    raise_err(v, err);
 }
@@ -2424,7 +2429,6 @@ __global__ void __launch_bounds__(CB) k_prim2cons(ViewT<R> v){
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
    if( i >= np ) return;
-   const int N = v.Ncell;
    int c = b.c0 + i;
    const DiskParams &P = v.dp[b.disk];
    int j = b.j, k = b.k;
@@ -2437,7 +2441,7 @@ __global__ void __launch_bounds__(CB) k_prim2cons(ViewT<R> v){
    double dV = dV_of(rj[j], rj[j-1], dph, zk[k], zk[k-1]);
    double prim[Q], cons[Q];
 #pragma unroll
-   for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[q*N+c];
+   for( int q=0 ; q<Q ; ++q ) prim[q] = (double)v.prim[AT(q, c)];
    bool done = false;
    if constexpr ( NC == 8 && sizeof(R) == sizeof(double) ){
       if( P.gr ){                   /* calc_cons with grmhd2 at the centroid */
@@ -2451,7 +2455,7 @@ __global__ void __launch_bounds__(CB) k_prim2cons(ViewT<R> v){
    }
    if( !done ) prim2cons<Q,NC,double>(P, prim, cons, r, get_om(P, r), dV);
 #pragma unroll
-   for( int q=0 ; q<Q ; ++q ) v.cons[q*N+c] = cons[q];
+   for( int q=0 ; q<Q ; ++q ) v.cons[AT(q, c)] = cons[q];
    raise_err(v, err);
 }
 
@@ -2462,7 +2466,6 @@ __global__ void __launch_bounds__(CB) k_wcell(ViewT<R> v){
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
    if( i >= np ) return;
-   const int N = v.Ncell;
    int c0 = b.c0, c = c0 + i;
    int cp = c0 + (i+1 == np ? 0 : i+1);
    const DiskParams &P = v.dp[b.disk];
@@ -2475,10 +2478,10 @@ __global__ void __launch_bounds__(CB) k_wcell(ViewT<R> v){
          const double *rj = v.rj + P.rj0 + 1, *zk = v.zk + P.zk0 + 1;
          double x[3] = {centroid_r(rj[j], rj[j-1]), 0.0, centroid_z(zk[k], zk[k-1])};
          double pc[Q], pr[Q];
-         for( int q=0 ; q<Q ; ++q ){ pc[q] = (double)v.prim[q*N + c]; pr[q] = (double)v.prim[q*N + cp]; }
+         for( int q=0 ; q<Q ; ++q ){ pc[q] = (double)v.prim[AT(q, c)]; pr[q] = (double)v.prim[AT(q, cp)]; }
          w = .5*(gr_omega_at(P, pc, x) + gr_omega_at(P, pr, x));
       }
-   }else if( P.mesh_motion ) w = .5*((double)v.prim[UPP*N + c] + (double)v.prim[UPP*N + cp]);
+   }else if( P.mesh_motion ) w = .5*((double)v.prim[AT(UPP, c)] + (double)v.prim[AT(UPP, cp)]);
    if( P.mesh_motion == 4 ){
       int j = b.j;
       const double *rj = v.rj + P.rj0 + 1;
@@ -2494,7 +2497,6 @@ __global__ void __launch_bounds__(CB) k_mindt(ViewT<R> v){
    const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
-   const int N = v.Ncell;
    int c0 = b.c0;
    int d = b.disk;
    const DiskParams &P = v.dp[d];
@@ -2518,21 +2520,21 @@ __global__ void __launch_bounds__(CB) k_mindt(ViewT<R> v){
       if constexpr ( NC == 8 && sizeof(R) == sizeof(double) ) gr = P.gr;
       if( gr ){                     /* mindt of grmhd2, grmhd2.c:748-832 */
          double pc[Q];
-         for( int q=0 ; q<Q ; ++q ) pc[q] = (double)v.prim[q*N+c];
+         for( int q=0 ; q<Q ; ++q ) pc[q] = (double)v.prim[AT(q, c)];
          double xp[3] = {rp, piph, zp}, xm[3] = {rm, phim, zm};
          double dtg = gr_mindt(P, v.gr_ann[a].m, pc, w, xp, xm, &err);
          if( dtg == dtg ) dtc = dtg;
       }else{
-         double vp = ((double)v.prim[UPP*N+c]-w)*r;
-         double cs = sqrt(P.gam*(double)v.prim[PPP*N+c]/(double)v.prim[RHO*N+c]);
+         double vp = ((double)v.prim[AT(UPP, c)]-w)*r;
+         double cs = sqrt(P.gam*(double)v.prim[AT(PPP, c)]/(double)v.prim[AT(RHO, c)]);
          if constexpr ( NC == 8 ){               /* mhd.c:452-486: fast speed */
-            double Br = v.prim[BRR*N+c], Bp = v.prim[BPP*N+c], Bz = v.prim[BZZ*N+c];
-            double b2 = (Br*Br+Bp*Bp+Bz*Bz)/(double)v.prim[RHO*N+c];
+            double Br = v.prim[AT(BRR, c)], Bp = v.prim[AT(BPP, c)], Bz = v.prim[AT(BZZ, c)];
+            double b2 = (Br*Br+Bp*Bp+Bz*Bz)/(double)v.prim[AT(RHO, c)];
             cs = sqrt(cs*cs + b2);
          }
-         double maxvr = cs + fabs((double)v.prim[URR*N+c]);
+         double maxvr = cs + fabs((double)v.prim[AT(URR, c)]);
          double maxvp = cs + fabs(vp);
-         double maxvz = cs + fabs((double)v.prim[UZZ*N+c]);
+         double maxvz = cs + fabs((double)v.prim[AT(UZZ, c)]);
          double dtr = (rp-rm)/maxvr;
          double dtp = (.5*(rp+rm))*get_dp(piph, phim, P.Pmax, &err)/maxvp;
          double dtz = (zp-zm)/maxvz;
@@ -2542,7 +2544,7 @@ __global__ void __launch_bounds__(CB) k_mindt(ViewT<R> v){
          if( P.visc ){
             double pc[Q];
 #pragma unroll
-            for( int q=0 ; q<Q ; ++q ) pc[q] = (double)v.prim[q*N+c];
+            for( int q=0 ; q<Q ; ++q ) pc[q] = (double)v.prim[AT(q, c)];
             dtm = visc_dt_limit(P, pc, r, dtm, rp, rm, zp, zm, get_dp(piph, phim, P.Pmax, &err));
          }
          if( dtm == dtm ) dtc = dtm;

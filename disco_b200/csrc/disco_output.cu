@@ -41,13 +41,12 @@ template<class R>
 __global__ void k_pack_rows(ViewT<R> v, size_t c0, size_t n, int Q, int F, int mode, double *out){
    size_t t = blockIdx.x*(size_t)blockDim.x + threadIdx.x;
    if( t >= n ) return;
-   const size_t N = v.Ncell;
-   size_t c = c0 + t;
+   const size_t c = c0 + t;
    int ncol = mode == ROWS_CELLS ? Q + F + 1 : Q + 2;
    double *o = out + t*ncol;
-   for( int q=0 ; q<Q ; ++q ) o[q] = (double)v.prim[q*N + c];
+   for( int q=0 ; q<Q ; ++q ) o[q] = (double)v.prim[at_rows(Q, q, c)];
    if( mode == ROWS_CELLS ){
-      for( int s=0 ; s<F ; ++s ) o[Q+s] = v.ct ? v.Phi[s*N + c] : 0.0;
+      for( int s=0 ; s<F ; ++s ) o[Q+s] = v.ct ? v.Phi[at_rows(v.nfs, s, c)] : 0.0;
       o[Q+F] = v.piph[c];
    }else{
       o[Q] = v.piph[c];
