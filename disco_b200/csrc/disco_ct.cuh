@@ -77,7 +77,7 @@ __device__ __forceinline__ void ct_over_runs(const ViewT<R> &v, const int *cons,
 }
 
 template<class R>
-__global__ void __launch_bounds__(CB) k_ct_edges(ViewT<R> v){
+__global__ void __launch_bounds__(CB, MB_CT_EDGES) k_ct_edges(ViewT<R> v){
    const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;
@@ -149,7 +149,7 @@ __device__ __forceinline__ int ct_prev(const ViewT<R> &v, int a, int c){
 }
 
 template<class R>
-__global__ void __launch_bounds__(FB) k_ct_faces(ViewT<R> v){
+__global__ void __launch_bounds__(FB, MB_CT_FACES) k_ct_faces(ViewT<R> v){
    const FaceBlk b = v.fblk[blockIdx.x];
    int t = b.x;
    bool zf = b.dim == 2;
@@ -378,7 +378,7 @@ __device__ __forceinline__ void ct_line_step(const ViewT<R> &v, const DiskParams
 }
 
 template<class R>
-__global__ void __launch_bounds__(CB) k_ct_line(ViewT<R> v){
+__global__ void __launch_bounds__(CB, MB_CT_LINE) k_ct_line(ViewT<R> v){
    __shared__ LineAnn A[3][3];
    __shared__ int s_o[4];
    const CellBlk b = v.cblk[blockIdx.x];
@@ -443,7 +443,7 @@ __device__ __forceinline__ double ct_line_terms(const ViewT<R> &v, double S, int
  * make_edge_adjust), then (first substep) move_cells / clean_pi / calc_dp
  * as k_update does without CT */
 template<class R>
-__global__ void __launch_bounds__(CB) k_ct_update(ViewT<R> v, int first){
+__global__ void __launch_bounds__(CB, MB_CT_UPDATE) k_ct_update(ViewT<R> v, int first){
    const CellBlk b = v.cblk[blockIdx.x];
    int a = b.x, i = b.y + threadIdx.x;
    int np = b.np;

@@ -107,13 +107,30 @@ namespace disco {
 /* the grmhd2 (GR) instantiations of the step kernels: resident blocks per
  * SM measured on the config-3 torus (192 x 16 x 462 slice, Kerr a = 0.9)
  * for 2-6 blocks: 5 for the flux kernels and k_update (2-4 spill less but
- * hide less latency: 8.4-10.1 ms per step at 2-3 against 7.4 at 5), 6 for
- * k_begin and k_c2p */
+ * hide less latency: 8.4-10.1 ms per step at 2-3 against 7.4 at 5), 7 for
+ * k_begin and k_c2p (ms per step at 5, 6, 7, 8 blocks: 0.440 0.418 0.390 0.385
+ * and 0.770 0.723 0.695 0.713) */
 #ifndef MB_GR
 #define MB_GR 5
 #endif
+/* the CT kernels.  They gather a few values per cell or face through two
+ * dependent loads each, so more warps beat the few words that spill.  ms per
+ * step, FP64 on the MHD grid of 64 x 64 annuli and mixed on 384 x 32 of the 3D
+ * binary, at the compiler's register count and at 8 / 10 / 12 / 16 blocks:
+ *   k_ct_edges   0.254: 0.237 0.238 0.249  -     1.004: 1.184 0.998 0.884  -
+ *   k_ct_faces   0.221:  -    0.209 0.201 0.176  1.112:  -    1.508 1.355 1.113
+ *   k_ct_line    0.312: 0.338 0.308 0.279  -     2.503: 2.785 2.453 2.281  -
+ *   k_ct_update  0.228: 0.267  -    0.202 0.197  1.918: 2.250  -    1.662 1.664 */
+#ifdef DISCO_MIXED_TU
+#define MB_CT_EDGES 12
+#else
+#define MB_CT_EDGES 8
+#endif
+#define MB_CT_FACES 16
+#define MB_CT_LINE 12
+#define MB_CT_UPDATE 12
 #ifndef MB_GR_LIGHT
-#define MB_GR_LIGHT 6
+#define MB_GR_LIGHT 7
 #endif
 
 /* A block's work and the entries of its annulus or track, in one load: read
@@ -131,12 +148,12 @@ struct __align__(16) FaceBlk { int x, y;          /* track, first face within it
  * field are as consecutive as with each field in a row of its own, but all
  * fields of a cell lie within a few kB instead of Ncell apart.  The step
  * kernels wait on memory, and a gather over Q rows of hundreds of MB waits on
- * address translation as well: ms per step, rows -> tiles, k_grad, k_faces
- * and k_flux of 32 disks of the 3D binary (mixed) 2.187 -> 1.884, 2.511 ->
- * 2.294 and 3.367 -> 3.007, the step 22.1 -> 20.6; 64 ragged disks FP64 4.288
- * -> 4.117, GRMHD torus 6.262 -> 5.971, one small disk 0.178 -> 0.175.  Tiles
- * of 128 are 0.2-0.4% slower; prim with its slopes, and cons with RKcons, in
- * one array each 0.5% slower than apart. */
+ * address translation as well: ms per step, rows -> tiles, on 384 x 32 annuli
+ * of the 3D binary (mixed) k_grad 2.187 -> 1.884, k_faces 2.511 -> 2.294,
+ * k_flux 3.367 -> 3.007, the step 22.1 -> 20.6; 64 ragged disks FP64 4.288 ->
+ * 4.117, GRMHD torus 6.262 -> 5.971, one small disk 0.178 -> 0.175.  Tiles of
+ * 128 are 0.2-0.4% slower; prim with its slopes, and cons with RKcons, in one
+ * array each 0.5% slower than apart. */
 #define TILE 32
 __host__ __device__ __forceinline__ size_t at_rows(int L, int q, unsigned c){
    return (size_t)(c & ~(TILE-1u))*(L-1) + c + q*TILE;
@@ -517,10 +534,10 @@ __device__ __forceinline__ int gallop_lb(int lo, int hi, int g, Pr p){
 /* The PLM face slopes S_q of plm_trans (plm.c:82-89).  In the mixed build all
  * loads come before the first store: the compiler may not move a load over a
  * store that might alias it, so loaded and stored field by field the fields
- * are Q round trips to memory in a row (k_faces, 32 disks of binary_nz:
- * 2.81 -> 2.51 ms per step; 64 disks of 5k..100k cells 0.570 -> 0.530).  FP64
- * keeps the round trips: Q slopes of 64 bits do not fit in the registers that
- * 16 blocks per SM leave a thread, and fewer blocks cost more than that
+ * are Q round trips to memory in a row (k_faces, ms per step: 384 x 32 annuli
+ * of the 3D binary 2.81 -> 2.51, 64 disks of 5k..100k cells 0.570 -> 0.530).
+ * FP64 keeps the round trips: Q slopes of 64 bits do not fit in the registers
+ * that 16 blocks per SM leave a thread, and fewer blocks cost more than that
  * (0.782 field by field, 0.911 together, 1.014 together at 10 blocks). */
 template<int Q, class R>
 __device__ __forceinline__ void face_slopes(const ViewT<R> &v, int cL, int cR, R dpL, R dpR, R dxL, R dxR, int f){
@@ -1017,7 +1034,8 @@ __device__ __forceinline__ QVec<Q,R> phi_face_flux_visc(const ViewT<R> &v, const
  * first (RK = 0) these are x itself, bit for bit, unless not finite.  Every
  * row is loaded before the first is stored (see face_slopes): k_update, ms per
  * step, 64 disks 1.031 -> 0.996 (mixed 1.009 -> 0.940), MHD 64x64 annuli
- * 0.637 -> 0.599; k_ct_update of 32 disks of binary_nz 2.147 -> 1.870. */
+ * 0.637 -> 0.599; k_ct_update of 384 x 32
+ * annuli of the 3D binary 2.147 -> 1.870. */
 template<int M>
 __device__ __forceinline__ void rk_start(const double *x, double *RKx, int L, int c, int first, double *x0){
 #pragma unroll

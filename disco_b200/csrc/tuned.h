@@ -21,8 +21,11 @@
  *          k_c2p        0.5651   0.4731   0.4832   0.4763   0.5304   -> 8
  *
  * k_faces of the mixed build since loads all its fields before it stores one
- * and takes 12 (0.530 at 16, 0.530 at 12 here; 2.652 and 2.509 on 32 disks of
- * the 3D binary).
+ * and takes 12 (0.530 at 16, 0.530 at 12 here; 2.652 and 2.509 on 384 x 32
+ * annuli of the 3D binary).  With the fields of a cell in one tile, the mixed
+ * build's k_gradr takes 12 (0.399 at 16, 0.383 at 12, 0.425 at 10) and k_flux_r
+ * 14 (0.516 at 12, 0.481 at 14, 0.525 at 10); the others stay the fastest of
+ * the values on either side.
  *
  * Values given with -D on the command line win.
  */
@@ -41,10 +44,10 @@
 #define MB_FACES 12
 #endif
 #ifndef MB_GRAD
-#define MB_GRAD 16
+#define MB_GRAD 12
 #endif
 #ifndef MB_FLUX
-#define MB_FLUX 12
+#define MB_FLUX 14
 #endif
 #ifndef MB_UPDATE
 #define MB_UPDATE 8

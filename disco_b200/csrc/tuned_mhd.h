@@ -18,12 +18,18 @@
  *          k_update     2.1891   2.0595   1.9458   1.8913   1.9089   2.0669   2.3853   -> 7
  *          k_c2p        1.9393   1.5485   1.3977   1.2502   1.1611   1.1900   1.2116   -> 8
  *
+ * With the fields of a cell in one tile and both directions in one k_flux
+ * launch, FP64 k_flux takes 7 (3D MHD grid of 64 x 64 annuli: 0.868 at 5, 0.865
+ * at 6, 0.834 at 7) and the mixed k_begin 10 (384 x 32 annuli of the 3D binary:
+ * 0.487 at 12, 0.480 at 10); the others stay the fastest of the values on
+ * either side.
+ *
  * Values given with -D on the command line win.
  */
 #pragma once
 #ifdef DISCO_MIXED_TU
 #ifndef MB_MHD_BEGIN
-#define MB_MHD_BEGIN 12
+#define MB_MHD_BEGIN 10
 #endif
 #ifndef MB_MHD_GRAD
 #define MB_MHD_GRAD 12
@@ -45,7 +51,7 @@
 #define MB_MHD_GRAD 8
 #endif
 #ifndef MB_MHD_FLUX
-#define MB_MHD_FLUX 5
+#define MB_MHD_FLUX 7
 #endif
 #ifndef MB_MHD_UPDATE
 #define MB_MHD_UPDATE 5
