@@ -59,8 +59,8 @@ def peaks():
 # the ragged8 workload (1,049,795 cells, 2,089,252 r-faces), from an ncu
 # capture of k_update and k_flux_t on that workload: (bytes, units the
 # launch processed)
-DRAM_UPDATE_RAGGED8 = (289.8e6 + 53.7e6, 1049795)
-DRAM_FLUX_RAGGED8 = (216.2e6 + 72.5e6, 2089252)
+DRAM_UPDATE_RAGGED8 = (282.0e6 + 76.0e6, 1049795)
+DRAM_FLUX_RAGGED8 = (217.2e6 + 74.7e6, 2089252)
 
 
 def kernel_bytes(name, first, N, Nf, Na, nreal=0):
