@@ -992,9 +992,9 @@ def ragged_leg(args, local, stream, barrier, allmax, rank, world):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one k_update launch of the
-# mixed form on the config-4 slab of 12 z layers (4,995,072 cells with
+# mixed form on the config-4 slab of 8 z layers (3,746,304 cells with
 # ghosts), from an ncu capture: (bytes, cells of that slab)
-DRAM_UPDATE_C4 = (1244454144 + 640664832, 4995072)
+DRAM_UPDATE_C4 = (1244454144 + 640664832, 3746304)
 
 
 def run_ours(args, world, rank, local):
@@ -1049,7 +1049,7 @@ def run_ours(args, world, rank, local):
             if dom != "k_update" or DRAM_UPDATE_C4 is None:
                 return None, None
             bb, cells = DRAM_UPDATE_C4
-            return bb / cells * ncell, ("ncu capture of one k_update launch on the 12-layer config-4 "
+            return bb / cells * ncell, ("ncu capture of one k_update launch on the 8-layer config-4 "
                                         "slab, scaled by the cells processed")
         b_step = B_ALG_MHD_CT["mixed"]
     else:
