@@ -1157,16 +1157,6 @@ extern "C" int disco_batch_run(disco_batch *b, int nsteps){
    if( !b || nsteps < 0 ) return DISCO_ERR_ARG;
    if( !b->have_cells ) return DISCO_ERR_STATE;
    CK(cudaSetDevice(b->device));
-   /* captured by the caller, to be replayed after an upload perhaps: the
-    * steps themselves, which look for their faces (launch_step_qt), not the
-    * graph of the step that keeps them */
-   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-   CK(cudaStreamIsCapturing(b->stream, &cap));
-   if( cap != cudaStreamCaptureStatusNone ){
-      for( int n=0 ; n<nsteps ; ++n ) launch_step(b, 1);
-      CK(cudaGetLastError());
-      return DISCO_OK;
-   }
    /* the captured step takes the kept faces as given: the first step after an
     * upload, which builds them, is launched as it is */
    if( nsteps > 0 && b->sched == DISCO_SCHED_KERNELS && b->timestep_mode == 0 && !b->topo_known ){
