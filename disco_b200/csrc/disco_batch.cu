@@ -1157,6 +1157,13 @@ extern "C" int disco_batch_run(disco_batch *b, int nsteps){
    if( !b || nsteps < 0 ) return DISCO_ERR_ARG;
    if( !b->have_cells ) return DISCO_ERR_STATE;
    CK(cudaSetDevice(b->device));
+   /* a caller's capture takes no graph launch: refused before anything of the
+    * run is captured */
+   if( nsteps > 0 ){
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      CK(cudaStreamIsCapturing(b->stream, &cap));
+      if( cap != cudaStreamCaptureStatusNone ) return DISCO_ERR_CUDA;
+   }
    /* the captured step takes the kept faces as given: the first step after an
     * upload, which builds them, is launched as it is */
    if( nsteps > 0 && b->sched == DISCO_SCHED_KERNELS && b->timestep_mode == 0 && !b->topo_known ){
