@@ -1141,6 +1141,10 @@ extern "C" int disco_batch_timestep(disco_batch *b, const double *dt){
    if( !b->have_cells ) return DISCO_ERR_STATE;
    CK(cudaSetDevice(b->device));
    if( dt ){                        /* by value with the launch: no copy, no wait */
+      /* a caller's capture would step with this dt at every replay: refused */
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      CK(cudaStreamIsCapturing(b->stream, &cap));
+      if( cap != cudaStreamCaptureStatusNone ) return DISCO_ERR_CUDA;
       for( int d0=0 ; d0<b->ndisk ; d0+=DtChunk::N ){
          DtChunk ch;
          ch.n = b->ndisk - d0 < DtChunk::N ? b->ndisk - d0 : DtChunk::N;

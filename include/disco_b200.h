@@ -210,6 +210,9 @@ int disco_batch_mindt(disco_batch *b, double *dt);
  * One full step of every disk: timestep() (timestep.c:7-45) with the given
  * per-disk dt (NULL = use the dt that the last mindt/step left on the
  * device, i.e. getmindt of the current state, with no host round trip).
+ * A caller may capture the call with dt = NULL in a CUDA graph and replay it
+ * on later states; with a dt it fails while the batch's stream is captured
+ * (DISCO_ERR_CUDA), as disco_batch_run does.
  */
 int disco_batch_timestep(disco_batch *b, const double *dt);
 
