@@ -1130,6 +1130,25 @@ static void launch_step(disco_batch *b, int use_next){
    else launch_step_t(b, b->vd, use_next);
 }
 
+/* calls that a caller's stream capture does not take; a refused query leaves
+ * no error behind for the next call to find */
+static int not_captured(disco_batch *b){
+   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+   if( cudaStreamIsCapturing(b->stream, &cap) != cudaSuccess ){
+      cudaGetLastError();
+      return DISCO_ERR_CUDA;
+   }
+   return cap == cudaStreamCaptureStatusNone ? DISCO_OK : DISCO_ERR_CUDA;
+}
+
+/* what the launches of a step returned; a refused step has built no faces */
+static int step_status(disco_batch *b){
+   const cudaError_t e = cudaGetLastError();
+   if( e != cudaSuccess ) b->topo_known = 0;
+   CK(e);
+   return DISCO_OK;
+}
+
 /* the dt of up to N disks, a kernel argument */
 struct DtChunk { enum { N = 64 }; int n; double dt[N]; };
 __global__ void k_set_dt(DiskState *ds, DtChunk ch){
@@ -1142,9 +1161,8 @@ extern "C" int disco_batch_timestep(disco_batch *b, const double *dt){
    CK(cudaSetDevice(b->device));
    if( dt ){                        /* by value with the launch: no copy, no wait */
       /* a caller's capture would step with this dt at every replay: refused */
-      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-      CK(cudaStreamIsCapturing(b->stream, &cap));
-      if( cap != cudaStreamCaptureStatusNone ) return DISCO_ERR_CUDA;
+      const int s = not_captured(b);
+      if( s ) return s;
       for( int d0=0 ; d0<b->ndisk ; d0+=DtChunk::N ){
          DtChunk ch;
          ch.n = b->ndisk - d0 < DtChunk::N ? b->ndisk - d0 : DtChunk::N;
@@ -1153,8 +1171,7 @@ extern "C" int disco_batch_timestep(disco_batch *b, const double *dt){
       }
    }
    launch_step(b, 1);
-   CK(cudaGetLastError());
-   return DISCO_OK;
+   return step_status(b);
 }
 
 extern "C" int disco_batch_run(disco_batch *b, int nsteps){
@@ -1164,15 +1181,15 @@ extern "C" int disco_batch_run(disco_batch *b, int nsteps){
    /* a caller's capture takes no graph launch: refused before anything of the
     * run is captured */
    if( nsteps > 0 ){
-      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-      CK(cudaStreamIsCapturing(b->stream, &cap));
-      if( cap != cudaStreamCaptureStatusNone ) return DISCO_ERR_CUDA;
+      const int s = not_captured(b);
+      if( s ) return s;
    }
    /* the captured step takes the kept faces as given: the first step after an
     * upload, which builds them, is launched as it is */
    if( nsteps > 0 && b->sched == DISCO_SCHED_KERNELS && b->timestep_mode == 0 && !b->topo_known ){
       launch_step(b, 1);
-      CK(cudaGetLastError());
+      const int s = step_status(b);
+      if( s ) return s;
       nsteps--;
    }
    if( !b->graph && nsteps > 0 ){
@@ -1420,7 +1437,8 @@ extern "C" int disco_batch_kernel_times(disco_batch *b, float *ms, const char **
    ev.push_back(e0);
    launch_step(b, 1);
    b->tape = NULL; b->tape_names = NULL;
-   CK(cudaGetLastError());
+   const int s = step_status(b);
+   if( s ) return s;
    CK(cudaStreamSynchronize(b->stream));
    int n = (int)nm.size();
    if( n > cap ) n = cap;
