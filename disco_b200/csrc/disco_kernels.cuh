@@ -1327,6 +1327,8 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
    else if( first ){                /* a ghost's cons is not evolved: its snapshot alone */
       double x0[Q];
       rk_start<Q>(v.cons, v.RKcons, Q, c, first, x0);
+#pragma unroll
+      for( int q=0 ; q<Q ; ++q ) if( !isfinite(x0[q]) ) v.cons[AT(q, c)] = x0[q];   /* inf is NaN by the average */
    }
    /* the move follows in k_c2p (or k_ct_update) */
    raise_err(v, err);
