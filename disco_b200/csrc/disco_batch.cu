@@ -669,27 +669,43 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
          if( b->zg_pairs.size() > first )
             b->zg_chains.push_back(make_int2((int)first, (int)(b->zg_pairs.size() - first)));
       };
+      /* sides s0 and s0+1 of a column of n annuli, ga and gb of them ghosts: a
+       * chain each, which run side by side; one chain, layer by layer, where
+       * a mirrored side's source is one of the other side's ghosts (fewer
+       * real annuli than ghost layers) */
+      auto column = [&](int s0, int n, int ga, int gb, auto annulus){
+         const int m0 = smode[s0], m1 = smode[s0+1];
+         auto lower = [&](int l){
+            const int x = ga-1-l, x1 = side_mirror(m0) ? 2*ga-x-1 : x+1;
+            pair_of(annulus(x), annulus(x1), flags(s0));
+         };
+         auto upper = [&](int l){
+            const int x = n-gb+l, x1 = side_mirror(m1) ? 2*(n-gb)-x-1 : x-1;
+            pair_of(annulus(x), annulus(x1), flags(s0+1));
+         };
+         const int na = side_copies(m0) ? ga : 0, nb = side_copies(m1) ? gb : 0, real = n - ga - gb;
+         size_t first = b->zg_pairs.size();
+         if( na && nb && ((side_mirror(m0) && real < na) || (side_mirror(m1) && real < nb)) ){
+            for( int l=0 ; l<na || l<nb ; ++l ){ if( l < na ) lower(l); if( l < nb ) upper(l); }
+            close(first);
+            return;
+         }
+         for( int l=0 ; l<na ; ++l ) lower(l);
+         close(first);
+         first = b->zg_pairs.size();
+         for( int l=0 ; l<nb ; ++l ) upper(l);
+         close(first);
+      };
       b->zg_off.push_back(0);
       for( int d=0 ; d<ndisk ; ++d ){
          const DiskParams &D = b->dparams[d];
          for( int k=0 ; k<D.Nz ; ++k ){
-            int base = D.ann0 + D.Nr*k;
+            const int base = D.ann0 + D.Nr*k;
             /* a z ghost layer of a fixed z side ends fixed (the z pass runs
              * after the r copies), so its r ghosts need no copy */
             if( (k < D.NgZa && smode[2] == SIDE_FIXED) || (k >= D.Nz - D.NgZb && smode[3] == SIDE_FIXED) )
                continue;
-            size_t first = b->zg_pairs.size();
-            if( side_copies(smode[0]) ) for( int l=0 ; l<D.NgRa ; ++l ){
-               int j = D.NgRa-1-l, j1 = side_mirror(smode[0]) ? 2*D.NgRa-j-1 : j+1;
-               pair_of(base+j, base+j1, flags(0));
-            }
-            close(first);
-            first = b->zg_pairs.size();
-            if( side_copies(smode[1]) ) for( int l=0 ; l<D.NgRb ; ++l ){
-               int j = D.Nr-D.NgRb+l, j1 = side_mirror(smode[1]) ? 2*(D.Nr-D.NgRb)-j-1 : j-1;
-               pair_of(base+j, base+j1, flags(1));
-            }
-            close(first);
+            column(0, D.Nr, D.NgRa, D.NgRb, [&](int j){ return base + j; });
          }
       }
       if( smode[1] == SIDE_ZG_DIODE_PHIWIN ){
@@ -712,20 +728,8 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
       for( int d=0 ; d<ndisk ; ++d ){
          const DiskParams &D = b->dparams[d];
          if( D.Nz < 2 || params[d].Z_Periodic ) continue;
-         for( int j=0 ; j<D.Nr ; ++j ){
-            size_t first = b->zg_pairs.size();
-            if( side_copies(smode[2]) ) for( int l=0 ; l<D.NgZa ; ++l ){
-               int k = D.NgZa-1-l, k1 = side_mirror(smode[2]) ? 2*D.NgZa-k-1 : k+1;
-               pair_of(D.ann0 + j + D.Nr*k, D.ann0 + j + D.Nr*k1, flags(2));
-            }
-            close(first);
-            first = b->zg_pairs.size();
-            if( side_copies(smode[3]) ) for( int l=0 ; l<D.NgZb ; ++l ){
-               int k = D.Nz-D.NgZb+l, k1 = side_mirror(smode[3]) ? 2*(D.Nz-D.NgZb)-k-1 : k-1;
-               pair_of(D.ann0 + j + D.Nr*k, D.ann0 + j + D.Nr*k1, flags(3));
-            }
-            close(first);
-         }
+         for( int j=0 ; j<D.Nr ; ++j )
+            column(2, D.Nz, D.NgZa, D.NgZb, [&](int k){ return D.ann0 + j + D.Nr*k; });
       }
       b->zg_off.push_back((int)b->zg_chains.size());
       size_t sm = 0;
