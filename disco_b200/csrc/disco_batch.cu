@@ -810,7 +810,10 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
       v.pE = ralloc(N); v.pB = ralloc(N);
       v.fEt = ralloc(face); v.fBt = ralloc(face);
       v.fX = dalloc<double>(b, face);
-      v.fPhi = dalloc<double>(b, face);
+      /* the face slopes are read last by k_grad, before any of these two is
+       * written, and are written next after k_c2p has read fPhi: 16 of their
+       * Q values' 36 or 72 bytes per face */
+      v.fPhi = (double *)v.fS + face;
       v.fFlip = dalloc<unsigned char>(b, face);
       if( ct == 2 ){
          v.pEr = ralloc(N); v.pBz = ralloc(N);
@@ -830,7 +833,7 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
             b->d_zpole = dupload(b, b->zpole);
          }
          if( b->any_3d ){
-            v.frk = dalloc<int>(b, 2*(size_t)face);
+            v.frk = (int *)v.fS;
             v.lineX = dalloc<double>(b, (size_t)b->line_ne);
             v.line_off = dupload(b, b->line_off);
          }

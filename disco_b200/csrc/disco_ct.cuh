@@ -426,16 +426,17 @@ __global__ void __launch_bounds__(CB, MB_CT_LINE) k_ct_line(ViewT<R> v){
 template<class R>
 __device__ __forceinline__ double ct_line_terms(const ViewT<R> &v, double S, int line, int tr,
                                                 int f, int slot, double sign){
-   const double *X = v.lineX + v.line_off[line];
-   const int *rank = v.frk + (size_t)slot*v.Nf;
+   const int l0 = v.line_off[line], ne = v.line_off[line+1] - l0;
+   const double *X = v.lineX + l0;
+   const int *frk = v.frk + (size_t)slot*v.Nf;
+   /* a face whose rank k_ct_line did not store (positions that are not finite,
+    * flagged there) holds anything */
+   auto rank = [&](int g){ const int e = frk[g]; return (unsigned)e < (unsigned)ne ? e : 0; };
    int f0 = v.tr_off[tr], f1 = v.tr_off[tr+1];
-   int hi = rank[f];
-   int lo = f == f0 ? 0 : rank[f-1] + 1;
+   int hi = rank(f);
+   int lo = f == f0 ? 0 : rank(f-1) + 1;
    for( int e=lo ; e<=hi ; ++e ) S += sign*X[e];
-   if( f == f0 ){
-      int ne = v.line_off[line+1] - v.line_off[line];
-      for( int e=rank[f1-1]+1 ; e<ne ; ++e ) S += sign*X[e];
-   }
+   if( f == f0 ) for( int e=rank(f1-1)+1 ; e<ne ; ++e ) S += sign*X[e];
    return S;
 }
 

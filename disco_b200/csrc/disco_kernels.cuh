@@ -226,7 +226,8 @@ struct ViewT {
     * the cell that ends the face, and lineX[line_off[l] + e] the E_phi dl dt of merged edge e of line l. */
    int ct, nfs;
    double *Phi, *RKPhi, *fX;            /* the face fluxes stay FP64 in both forms */
-   double *fPhi;                        /* each face's flux after the second substep's update */
+   double *fPhi;                        /* each face's flux after the second substep's update
+                                         * (fPhi and frk lie in fS, which no kernel reads meanwhile) */
    /* grmhd2: the metric at the fixed points where the step evaluates it
     * (k_gr_tables; NULL for the Newtonian modules) */
    GRAnn *gr_ann;
