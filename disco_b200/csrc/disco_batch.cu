@@ -32,9 +32,9 @@ static int cuda_status(cudaError_t e){
 static void *dalloc_bytes(disco_batch *b, size_t bytes){
    void *p = NULL;
    if( bytes == 0 ) bytes = 8;
-   if( cudaMalloc(&p, bytes) != cudaSuccess ) return NULL;
-   cudaMemset(p, 0, bytes);
-   b->allocs.push_back(p);
+   if( cudaMalloc(&p, bytes) != cudaSuccess ){ p = NULL; cudaGetLastError(); }
+   else cudaMemset(p, 0, bytes);
+   b->allocs.push_back(p);          /* NULL too: disco_batch_create looks for it before any launch */
    return p;
 }
 template<class T>
