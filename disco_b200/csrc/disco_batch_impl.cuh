@@ -72,7 +72,9 @@ struct disco_batch {
    cudaStream_t own_stream;
    std::vector<cudaEvent_t> *tape;       /* non-NULL: record an event after each launch */
    std::vector<const char *> *tape_names;
-   cudaGraphExec_t graph;
+   cudaGraphExec_t graph;    /* the step that takes the kept faces as given (any step without kept faces) */
+   cudaGraphExec_t graph_up; /* the step after an upload, which builds them: from the second such run on */
+   int up_runs;
    int have_cells;
    int topo_known;           /* the device's topo flag is set once the queued work has run */
    int own_capture, general; /* disco_batch_run is capturing; the step in flight runs every pass */

@@ -35,3 +35,21 @@ def test_run_after_upload(base, over, prec, how):
         for _ in range(n):
             fresh.timestep()
         same(fresh.get_cells(), b.get_cells())
+
+
+@pytest.mark.parametrize("base,over", DISKS)
+def test_one_step_after_each_upload(base, over):
+    """The step after an upload is launched the first time and a graph of its own from then on."""
+    d = make_disk(base, over)
+    b, fresh = db.Batch([d]), db.Batch([d])
+    states = [moved_on(b, d)]
+    states += [b.get_cells(), states[0]]
+    for n in (1, 2, 1, 3):
+        for st in states:
+            fresh.set_cells(**st)
+            b.set_cells(**st)
+            assert b.mindt() == fresh.mindt()
+            b.run(n)
+            for _ in range(n):
+                fresh.timestep()
+            same(fresh.get_cells(), b.get_cells())
