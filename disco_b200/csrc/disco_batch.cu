@@ -1137,9 +1137,9 @@ extern "C" int disco_batch_mindt(disco_batch *b, double *dt){
    return *h_err ? read_err(b) : DISCO_OK;
 }
 
-static void launch_step(disco_batch *b, int use_next){
-   if( b->prec == DISCO_PREC_MIXED ) mixed_launch_step(b, use_next);
-   else launch_step_t(b, b->vd, use_next);
+static void launch_step(disco_batch *b){
+   if( b->prec == DISCO_PREC_MIXED ) mixed_launch_step(b);
+   else launch_step_t(b, b->vd);
 }
 
 /* calls that a caller's stream capture does not take; a refused query leaves
@@ -1182,7 +1182,7 @@ extern "C" int disco_batch_timestep(disco_batch *b, const double *dt){
          k_set_dt<<<1, DtChunk::N, 0, b->stream>>>(b->vd.ds + d0, ch);
       }
    }
-   launch_step(b, 1);
+   launch_step(b);
    return step_status(b);
 }
 
@@ -1193,7 +1193,7 @@ static int capture_step(disco_batch *b, cudaGraphExec_t *out){
    cudaGraph_t g;
    CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
    b->own_capture = 1;
-   launch_step(b, 1);
+   launch_step(b);
    b->own_capture = 0;
    b->topo_known = known && b->sched == DISCO_SCHED_KERNELS;
    CK(cudaStreamEndCapture(b->stream, &g));
@@ -1219,7 +1219,7 @@ extern "C" int disco_batch_run(disco_batch *b, int nsteps){
     * on an MHD grid of 28 x 12 with constrained transport) */
    if( nsteps > 0 && b->sched == DISCO_SCHED_KERNELS && b->timestep_mode == 0 && !b->topo_known ){
       int s;
-      if( b->up_runs++ == 0 ) launch_step(b, 1);
+      if( b->up_runs++ == 0 ) launch_step(b);
       else{
          if( !b->graph_up && (s = capture_step(b, &b->graph_up)) ) return s;
          cudaGraphLaunch(b->graph_up, b->stream);
@@ -1465,7 +1465,7 @@ extern "C" int disco_batch_kernel_times(disco_batch *b, float *ms, const char **
    CK(cudaEventCreate(&e0));
    CK(cudaEventRecord(e0, b->stream));
    ev.push_back(e0);
-   launch_step(b, 1);
+   launch_step(b);
    b->tape = NULL; b->tape_names = NULL;
    const int s = step_status(b);
    if( s ) return s;

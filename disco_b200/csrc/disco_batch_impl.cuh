@@ -282,9 +282,8 @@ static void launch_substep(disco_batch *b, ViewT<R> v, int first, int last, doub
 
 /* timestep() as one cooperative launch of k_step (the counters zeroed first) */
 template<int Q, int NC, class R, int NQD>
-static void launch_persist_nq(disco_batch *b, const ViewT<R> &v, int use_next){
+static void launch_persist_nq(disco_batch *b, const ViewT<R> &v){
    PersistArgs pa = b->pargs;
-   pa.use_next = use_next;
    cudaMemsetAsync(b->d_pcnt, 0, b->pcnt_bytes, b->stream);
    cudaLaunchConfig_t cfg = {};
    cfg.gridDim = dim3((unsigned)b->pgrid);
@@ -300,12 +299,12 @@ static void launch_persist_nq(disco_batch *b, const ViewT<R> &v, int use_next){
    mark(b, "k_step");
 }
 template<int Q, int NC, class R>
-static void launch_persist(disco_batch *b, const ViewT<R> &v, int use_next){
+static void launch_persist(disco_batch *b, const ViewT<R> &v){
    if constexpr ( NC == 8 ){
-      if( b->nq == 18 ){ launch_persist_nq<Q,NC,R,18>(b, v, use_next); return; }
+      if( b->nq == 18 ){ launch_persist_nq<Q,NC,R,18>(b, v); return; }
    }
-   if( b->nq == 8 ) launch_persist_nq<Q,NC,R,8>(b, v, use_next);
-   else launch_persist_nq<Q,NC,R,5>(b, v, use_next);
+   if( b->nq == 8 ) launch_persist_nq<Q,NC,R,8>(b, v);
+   else launch_persist_nq<Q,NC,R,5>(b, v);
 }
 /* resident k_step CTAs per SM for the batch's instantiation */
 template<int Q, int NC, class R, int NQD>
@@ -323,10 +322,10 @@ static int persist_blocks_per_sm_t(const disco_batch *b){
 
 /* timestep() (timestep.c:7-45). */
 template<int Q, int NC, class R, bool GR = false>
-static void launch_step_qt(disco_batch *b, const ViewT<R> &v, int use_next){
+static void launch_step_qt(disco_batch *b, const ViewT<R> &v){
    if( b->sched == DISCO_SCHED_PERSISTENT ){
       b->topo_known = 0;            /* a launch that timed out leaves no list */
-      launch_persist<Q,NC,R>(b, v, use_next);
+      launch_persist<Q,NC,R>(b, v);
       return;
    }
    const bool fe = b->timestep_mode == 1;
@@ -361,11 +360,11 @@ static void launch_restart_t(disco_batch *b, const ViewT<R> &v){
    if( b->NC == 8 ) launch_restart_qt<9,8,R>(b, v); else launch_restart_qt<6,5,R>(b, v);
 }
 template<class R>
-static void launch_step_t(disco_batch *b, const ViewT<R> &v, int use_next){
+static void launch_step_t(disco_batch *b, const ViewT<R> &v){
    if constexpr ( sizeof(R) == sizeof(double) ){
-      if( b->gr ){ launch_step_qt<9,8,R,true>(b, v, use_next); return; }
+      if( b->gr ){ launch_step_qt<9,8,R,true>(b, v); return; }
    }
-   if( b->NC == 8 ) launch_step_qt<9,8,R>(b, v, use_next); else launch_step_qt<6,5,R>(b, v, use_next);
+   if( b->NC == 8 ) launch_step_qt<9,8,R>(b, v); else launch_step_qt<6,5,R>(b, v);
 }
 template<class R>
 static void launch_prim2cons_t(disco_batch *b, const ViewT<R> &v){
@@ -389,7 +388,7 @@ void mixed_launch_report(disco_batch *b);
 void mixed_launch_mindt(disco_batch *b);
 void mixed_launch_setup(disco_batch *b);
 void mixed_launch_restart(disco_batch *b);
-void mixed_launch_step(disco_batch *b, int use_next);
+void mixed_launch_step(disco_batch *b);
 void mixed_launch_prim2cons(disco_batch *b);
 void mixed_launch_faces(disco_batch *b);
 int mixed_prepare_zerograd(disco_batch *b);

@@ -2025,10 +2025,10 @@ __global__ void __launch_bounds__(ZG_T) k_zerograd(ViewT<R> v, const int2 *chain
 /* ------------------------------------------------------------------ per disk */
 /* Start of timestep(): planet_RK_copy, reset of the dt reduction. */
 template<class R>
-__device__ __forceinline__ void disk_begin_body(const ViewT<R> &v, int d, int use_next){
+__device__ __forceinline__ void disk_begin_body(const ViewT<R> &v, int d){
    DiskState &S = v.ds[d];
    const DiskParams &P = v.dp[d];
-   if( use_next ) S.dt = S.dt_next;
+   S.dt = S.dt_next;
    for( int p=0 ; p<P.npl ; ++p ){
       Planet &pl = S.pl[p];
       pl.RK_r = pl.r; pl.RK_phi = pl.phi; pl.RK_M = pl.M; pl.RK_omega = pl.omega; pl.RK_vr = pl.vr;
@@ -2128,7 +2128,7 @@ k_begin(ViewT<R> v, int first, int nI0, int ndisk){
    }
    const int d = ((int)blockIdx.x - nI0)*CB + threadIdx.x;
    if( d >= ndisk ) return;
-   if( first ) disk_begin_body<R>(v, d, 1);
+   if( first ) disk_begin_body<R>(v, d);
    else disk_mid_body<R>(v, d, 0.0, 1, 1);
 }
 

@@ -65,7 +65,7 @@ struct PersistArgs {
    const int *ndc;        /* per disk: cblk blocks */
    double *Qrz;
    const int *ann_blk0, *ann_nblk;
-   int bc, diag, use_next;
+   int bc, diag;
 };
 
 __device__ __forceinline__ int ld_acquire(const int *p){
@@ -223,7 +223,7 @@ __device__ __forceinline__ void persist_run(const ViewT<R> &v, const PersistArgs
    const int tid = threadIdx.x;
    const double dtfac = sub ? 0.5 : 1.0;
    switch( stage ){
-   case PS_DBEGIN:  if( tid == 0 ) disk_begin_body<R>(v, x, pa.use_next); break;
+   case PS_DBEGIN:  if( tid == 0 ) disk_begin_body<R>(v, x); break;
    case PS_BEGIN:   begin_body<Q,NC,R>(v, !sub, x); break;
    case PS_I0:      if( (tid >> 5) < n ) I0_body<R>(v, !sub, x + (tid >> 5), tid & 31); break;
    case PS_FACES:   faces_body<Q,R>(v, 1, !sub, x); break;
