@@ -113,6 +113,9 @@ namespace disco {
 #ifndef MB_GR
 #define MB_GR 5
 #endif
+#ifndef MB_GR_LIGHT
+#define MB_GR_LIGHT 7
+#endif
 /* the CT kernels.  They gather a few values per cell or face through two
  * dependent loads each, so more warps beat the few words that spill.  ms per
  * step, FP64 on the MHD grid of 64 x 64 annuli and mixed on 384 x 32 of the 3D
@@ -121,16 +124,21 @@ namespace disco {
  *   k_ct_faces   0.221:  -    0.209 0.201 0.176  1.112:  -    1.508 1.355 1.113
  *   k_ct_line    0.312: 0.338 0.308 0.279  -     2.503: 2.785 2.453 2.281  -
  *   k_ct_update  0.228: 0.267  -    0.202 0.197  1.918: 2.250  -    1.662 1.664 */
+#ifndef MB_CT_EDGES
 #ifdef DISCO_MIXED_TU
 #define MB_CT_EDGES 12
 #else
 #define MB_CT_EDGES 8
 #endif
+#endif
+#ifndef MB_CT_FACES
 #define MB_CT_FACES 16
+#endif
+#ifndef MB_CT_LINE
 #define MB_CT_LINE 12
+#endif
+#ifndef MB_CT_UPDATE
 #define MB_CT_UPDATE 12
-#ifndef MB_GR_LIGHT
-#define MB_GR_LIGHT 7
 #endif
 
 /* A block's work and the entries of its annulus or track, in one load: read
