@@ -115,11 +115,11 @@ static void launch_zerograd(disco_batch *b, const ViewT<R> &v){
    if( !b->bc_zerograd ) return;
    for( size_t g=0 ; g+1<b->zg_off.size() ; ++g ){
       int n = b->zg_off[g+1] - b->zg_off[g];
-      if( n > 0 ) k_zerograd<Q,R><<<n, ZG_T, b->zg_smem, b->stream>>>(v, b->d_zg_chains + b->zg_off[g],
-                                                                      b->d_zg_pairs, b->d_zg_side,
-                                                                      b->zg_diode, b->zg_omk);
+      if( n == 0 ) continue;
+      k_zerograd<Q,R><<<n, ZG_T, b->zg_smem, b->stream>>>(v, b->d_zg_chains + b->zg_off[g], b->d_zg_pairs,
+                                                          b->d_zg_side, b->zg_diode, b->zg_omk);
+      mark(b, "k_zerograd");
    }
-   mark(b, "k_zerograd");
 }
 template<int Q, class R>
 static int prepare_zerograd(disco_batch *b){
@@ -229,8 +229,11 @@ static void launch_substep(disco_batch *b, ViewT<R> v, int first, int last, doub
    v.move_c2p = first && !b->ct;
    cudaStream_t s = b->stream;
    unsigned ncb = (unsigned)b->cblk.size(), nfb = (unsigned)b->fblk.size();
-   const unsigned nI0 = build ? nblk((size_t)v.Nann, CB/32) : 0;
-   mark(b, "k_I0");                                    /* part of the next launch */
+   unsigned nI0 = build ? nblk((size_t)v.Nann, CB/32) : 0;
+   if( b->tape ){                   /* instrumented: a launch of its own, with its own time */
+      k_I0<R><<<nI0, CB, 0, s>>>(v);                   mark(b, "k_I0");
+      nI0 = 0;
+   }
    k_begin<Q,NC,R,GR><<<nI0 + nblk(b->ndisk, CB) + ncb, CB, 0, s>>>(v, first, (int)nI0, b->ndisk);
    mark(b, "k_begin");
    {  /* the same blocks in the order that keeps an annulus's three tracks together */

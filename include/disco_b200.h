@@ -361,7 +361,9 @@ int disco_batch_set_gr_dump(disco_batch *b, double *dev);
 /*
  * Run one full step with a CUDA event between every kernel launch and
  * return each launch's device time: ms[i] and the kernel's name in
- * names[i] (static strings), for i < *nlaunch (at most cap).  The
+ * names[i] (static strings), for i < *nlaunch (at most cap).  Every pass of
+ * the step runs; the search for each annulus's first cell past phi = 0, which
+ * a plain step does in blocks of k_begin, is a launch of its own (k_I0).  The
  * reference's profiler (profiler.c:188-206) labels the same phases.
  */
 int disco_batch_kernel_times(disco_batch *b, float *ms, const char **names, int cap, int *nlaunch);
