@@ -21,6 +21,8 @@ REF_LIB = os.path.join(HERE, "_ref", "c2p", "libc2p_ref.so")
 # the reference source tree the oracle builds compile; DISCO_REF overrides it
 REF_SRC = os.environ.get("DISCO_REF", "/root/reference")
 if not os.path.exists(os.path.join(REF_SRC, "paul.h")):
+    if "DISCO_REF" in os.environ:
+        raise FileNotFoundError("DISCO_REF=%s holds no reference sources (no paul.h)" % REF_SRC)
     REF_SRC = os.path.join(REF_SRC, "absent")      # a directory without the sources is no tree
 
 NPARAM = 64 * 8 + 64 + 64 * 64 + 64 + 2 * 64 + 2
