@@ -126,8 +126,11 @@ def kernel_bytes_mhd(name, first, N, Nfr, Nfz, mixed):
         return (Nfr + Nfz) * (8 + 3 * w + q * wr + 2 * wr) + N * (4 * q * wr + 2 * w)
     if name == "k_c2p":
         # cons (+carry), piph / dphi (moved in the first substep), the face
-        # fluxes rebuilt into the cell field, the prims written (+wiph last)
-        return N * (q * (w + ck) + 2 * w + phi + 3 * w + q * wr) + (0 if first else N * w)
+        # fluxes rebuilt into the cell field -- the cells' slots in the first
+        # substep, one flux per r and z face (fPhi) and the cells' phi-face
+        # slot in the second --, the prims written (+wiph last)
+        fluxes = N * phi if first else (Nfr + Nfz) * w + N * w
+        return N * (q * (w + ck) + 2 * w + 3 * w + q * wr) + fluxes + (0 if first else N * w)
     if name == "k_begin":
         return N * (2 * q * wr + w + (3 * w if first else 0))
     if name in ("k_gradr", "k_gradz"):
