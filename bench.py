@@ -377,11 +377,15 @@ def time_reference_c4(nsteps, max_workers=None):
 def run_reference(args, world, rank):
     if rank != 0:
         return
-    if args.workload == "config4":
-        v, cores, sample, _ = time_reference_c4(max(1, args.steps // 10))
-        nreal = C4_REAL_PER_LAYER * args.c4_nz
-    else:
-        v, cores, sample, nreal = time_reference(args.workload, max(1, args.steps // 4))
+    try:
+        if args.workload == "config4":
+            v, cores, sample, _ = time_reference_c4(max(1, args.steps // 10))
+            nreal = C4_REAL_PER_LAYER * args.c4_nz
+        else:
+            v, cores, sample, nreal = time_reference(args.workload, max(1, args.steps // 4))
+    except FileNotFoundError as ex:          # neither its sources nor a build of them
+        print(json.dumps({"impl": "reference", "unavailable": str(ex)}), flush=True)
+        return
     line = {"metric": METRIC, "value": v, "unit": "zone-updates/s", "n_gpus": args.gpus,
             "steps": args.steps, "warmup": args.warmup, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
