@@ -3,9 +3,9 @@
  * host <-> device state transfer, and the per-step launch sequence that
  * replaces timestep()/onestep() (timestep.c:7-45, onestep.c:84-229).
  *
- * One batch = one or more independent disks in one set of ragged SoA
- * arrays.  A substep is begin / I0 / faces / gradr / flux_r / flux_p /
- * update / c2p, a step two substeps plus three tiny per-disk kernels; the
+ * One batch = one or more independent disks in one set of ragged arrays
+ * (several fields in tiles, at_rows).  A substep is begin / faces / grad /
+ * flux / update / c2p, a step two substeps plus a closing kernel; the
  * multi-step driver captures one step in a CUDA graph and replays it with
  * dt left on the device by the previous step's fused getmindt.
  *
@@ -943,7 +943,7 @@ static cudaError_t xfer(const disco_batch *b, void *dst, const void *src, size_t
    return cudaStreamSynchronize(b->stream);
 }
 
-/* cell-major FP64 (Q per cell) host <-> SoA device of element type T: one
+/* cell-major FP64 (Q per cell) host <-> tiled device array of element type T: one
  * contiguous copy through a device staging array (DMA at full speed when the
  * host buffer is pinned), transposed on the device, one thread per cell.
  * The copies of a call are queued on the batch's stream one after another

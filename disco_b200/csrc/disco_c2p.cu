@@ -233,8 +233,11 @@ struct C2PSmem {
  * invariants, which only the recovery needs, are computed again afterwards
  * from a second (cached) read of the cell's cons and position.  The solve is
  * bound by the latency of its FP64 division chain, so resident warps matter
- * more than the few spills that 3 blocks of 256 per SM (80 registers) cost
- * in the set-up and recovery: measured 12% faster than 2 blocks. */
+ * more than the spills that 3 blocks of 256 per SM (80 registers) cost in the
+ * set-up and recovery.  us for 946,176 / 4,000,001 cells, warm start 1e-3 away,
+ * tail of 10: 2 blocks (126 registers, no spill) 300 / 1144, 3 blocks 262 / 1017,
+ * 4 blocks (64 registers, 612 B spilled) 259 / 1013; without a tail 242 / 888,
+ * 215 / 814, 209 / 805. */
 template<bool LEARNED, bool DUMP>
 __global__ void __launch_bounds__(C2P_BLOCK, 3)
 k_gr_c2p(GRParams P, long n, const double *__restrict__ cons, const double *__restrict__ x,

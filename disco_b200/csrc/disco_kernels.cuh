@@ -20,8 +20,8 @@
  *              (Np_a + Np_b of them, faces_alt.c:87-100).  Per disk the
  *              (Nr-1)*Nz r-tracks (tr_dim 1) come first, then the
  *              Nr*(Nz-1) z-tracks (tr_dim 2)
- *   faces      SoA: fL, fR (global cells), fLR, fphic, fdA, fdp (FP64),
- *              fS[q], fG[q] (R)
+ *   faces      one value each fL, fR (global cells), fLR, fphic, fdA, fdp (FP64);
+ *              in tiles, as the cells' fields, fS, fG (R)
  *   consume    consL[c] = face of the r-track outside c that consumes c in the
  *              merge; consR[c] = same for the track inside c (consZL/consZR:
  *              the z-tracks above / below c).  They give each
@@ -154,9 +154,10 @@ struct __align__(16) FaceBlk { int x, y;          /* track, first face within it
 /* Element (q, c) of an array of L fields over the cells or faces: tiles of
  * TILE cells, the fields of a tile one after another.  A warp's loads of a
  * field are as consecutive as with each field in a row of its own, but all
- * fields of a cell lie within a few kB instead of Ncell apart.  The step
- * kernels wait on memory, and a gather over Q rows of hundreds of MB waits on
- * address translation as well: ms per step, rows -> tiles, on 384 x 32 annuli
+ * fields of a cell lie within a few kB instead of Ncell apart, in hundreds of
+ * MB.  The step kernels wait on memory, the gathers most (which part of the
+ * wait the tiles remove, address translation or DRAM pages, was not
+ * measured): ms per step, rows -> tiles, on 384 x 32 annuli
  * of the 3D binary (mixed) k_grad 2.187 -> 1.884, k_faces 2.511 -> 2.294,
  * k_flux 3.367 -> 3.007, the step 22.1 -> 20.6; 64 ragged disks FP64 4.288 ->
  * 4.117, GRMHD torus 6.262 -> 5.971, one small disk 0.178 -> 0.175.  Tiles of
@@ -726,7 +727,6 @@ __device__ __forceinline__ void grad_body(const ViewT<R> &v, int bid){
    Runs Rin = {1,0,1,0}, Rout = {1,0,1,0};
    if( tin >= 0 ) Rin = cell_runs(v, cin, tin, c0, np, i, I0);
    if( tout >= 0 ) Rout = cell_runs(v, cout, tout, c0, np, i, I0);
-   const size_t Nf = v.Nf;
 #define ACC_RUN(s,e) for( int f=(s) ; f<=(e) ; ++f ){ R dA = (R)v.fdA[f]; \
       _Pragma("unroll") for( int q=0 ; q<Q ; ++q ) g[q] += v.fS[AT(q, f)]*dA; }
    ACC_RUN(Rin.s1, Rin.e1)
@@ -1237,7 +1237,6 @@ __device__ __forceinline__ void update_body(const ViewT<R> &v, int first, double
       Runs Rin = {1,0,1,0}, Rout = {1,0,1,0};
       if( j >= 1 ) Rin = cell_runs(v, v.consR, P.trr0 + (j-1) + (P.Nr-1)*k, c0, np, i, I0);
       if( j <= P.Nr-2 ) Rout = cell_runs(v, v.consL, P.trr0 + j + (P.Nr-1)*k, c0, np, i, I0);
-      const size_t Nf = v.Nf;
 #define ADD_RUN(s,e,sg) for( int f=(s) ; f<=(e) ; ++f ){ \
       _Pragma("unroll") for( int q=0 ; q<Q ; ++q ) addf(q, sg (double)v.fG[AT(q, f)]); }
       ADD_RUN(Rin.s1, Rin.e1, +)
