@@ -859,6 +859,7 @@ extern "C" int disco_batch_create(int device, const disco_modules *mods, int pre
       k_precompute<<<nblk(nx, 128), 128, 0, b->stream>>>(v);
       if( b->gr ) k_gr_tables<double><<<nblk(nx, 128), 128, 0, b->stream>>>(v);
       k_planet_trig<double><<<nblk(ndisk, 64), 64, 0, b->stream>>>(v, ndisk);
+      k_cons_init<double><<<(unsigned)b->cblk.size(), CB, 0, b->stream>>>(v);
    }
    /* the multi-kernel schedule is the default: on ragged64 the persistent
     * step measured 8.3 ms against 4.8 ms (FP64) and 7.2-7.9 against 3.9 ms

@@ -662,6 +662,25 @@ __global__ void __launch_bounds__(FB, MB_FACES) k_faces(ViewT<R> v, int with_slo
    faces_body<Q,R>(v, with_slopes, v.topo_reuse, blockIdx.x);
 }
 
+/* Set-up: every cell ends the first face of each of its tracks, until k_faces
+ * finds the one it does end.  A cell that ends none (a position that is not
+ * finite, in a first upload) then leaves its neighbour a run within the track
+ * (cell_runs), not one from face 0 of the batch. */
+template<class R>
+__global__ void __launch_bounds__(CB) k_cons_init(ViewT<R> v){
+   const CellBlk b = v.cblk[blockIdx.x];
+   const int i = b.y + threadIdx.x, j = b.j, k = b.k;
+   if( i >= b.np ) return;
+   const DiskParams &P = v.dp[b.disk];
+   const int c = b.c0 + i;
+   if( j <= P.Nr-2 ) v.consL[c] = v.tr_off[P.trr0 + j + (P.Nr-1)*k];
+   if( j >= 1 )      v.consR[c] = v.tr_off[P.trr0 + (j-1) + (P.Nr-1)*k];
+   if( P.Nz > 1 ){
+      if( k <= P.Nz-2 ) v.consZL[c] = v.tr_off[P.trz0 + j + P.Nr*k];
+      if( k >= 1 )      v.consZR[c] = v.tr_off[P.trz0 + j + P.Nr*(k-1)];
+   }
+}
+
 /* The faces of track t in which cell c (k-th edge from I0 of its annulus,
  * cell index i) is the head on its side, in face order: run 1 is
  * [s1, e1]; the I0 cell also heads the faces after the other annulus wraps,
